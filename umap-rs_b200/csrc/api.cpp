@@ -513,8 +513,7 @@ std::unique_ptr<umap_optimizer> optimizer_prepare_impl(std::unique_ptr<umap_mani
     compute_kept_edges(*o, K, true, true);
     log.mark("optimizer edge filtering + epochs_per_sample complete");
     const bool generic = o->metric_type == UMAP_METRIC_GENERIC;
-    build_sgd_layout(K.ptr.p, K.tail.p, K.eps.p, n, generic ? pick_chunk_generic(K.E) : 0, o->layout, s, nullptr,
-                     !generic);
+    build_sgd_layout(K.ptr.p, K.tail.p, K.eps.p, n, (uint32_t)dims, 0, generic, o->layout, s);
     log.mark("optimizer task layout complete");
   }
   if (log.on)
@@ -602,7 +601,7 @@ void step_epochs_impl(umap_optimizer& o, uint64_t n_ep, int output_metric = UMAP
     try {
       for (uint64_t epoch = o.current_epoch; epoch < o.current_epoch + n_ep; ++epoch) {
         const float alpha = o.initial_alpha * (1.0f - ((float)epoch / (float)o.total_epochs));  // :317
-        sgd_epoch(o.layout, live, snap, p, (uint32_t)epoch, alpha, s);
+        sgd_epoch(o.layout, live, snap, p, (uint32_t)epoch, alpha, epoch > o.current_epoch, s);
       }
     } catch (...) {
       cudaGraph_t g2 = nullptr;
@@ -624,7 +623,7 @@ void step_epochs_impl(umap_optimizer& o, uint64_t n_ep, int output_metric = UMAP
   } else {
     for (uint64_t epoch = o.current_epoch; epoch < o.current_epoch + n_ep; ++epoch) {
       const float alpha = o.initial_alpha * (1.0f - ((float)epoch / (float)o.total_epochs));  // :317
-      sgd_epoch(o.layout, live, snap, p, (uint32_t)epoch, alpha, s);
+      sgd_epoch(o.layout, live, snap, p, (uint32_t)epoch, alpha, epoch > o.current_epoch, s);
     }
   }
   UB_CUDA(cudaEventRecord(ev[1], s));
@@ -715,8 +714,8 @@ std::unique_ptr<umap_fitted> fit_impl(const umap_config& c, uint64_t n_samples, 
 }
 
 // ------------------------------------------------------------------ autotuning
-// Picks the SGD task length ("edges per thread") and the block shape by timing a few
-// epochs of each candidate on a scratch copy of the embedding.  Choices are cached per
+// Picks the SGD task length ("edges per thread") by timing two epochs of each candidate on a
+// scratch copy of the embedding.  Choices are cached per
 // problem size (vertices, edges in MiB units, dims) for the life of the process.
 struct TuneKey {
   uint64_t n, e_mib, dim;
@@ -725,7 +724,7 @@ struct TuneKey {
   }
 };
 std::mutex& g_tune_mu = *new std::mutex;
-std::map<TuneKey, std::pair<uint32_t, uint32_t>>& g_tuned = *new std::map<TuneKey, std::pair<uint32_t, uint32_t>>;
+std::map<TuneKey, uint32_t>& g_tuned = *new std::map<TuneKey, uint32_t>;
 
 void tune_layout(umap_optimizer& o, const KeptEdges& K) {
   cudaStream_t s = o.s();
@@ -737,13 +736,11 @@ void tune_layout(umap_optimizer& o, const KeptEdges& K) {
     std::lock_guard<std::mutex> lock(g_tune_mu);
     auto it = g_tuned.find(key);
     if (it != g_tuned.end()) {
-      build_sgd_layout(K.ptr.p, K.tail.p, K.eps.p, n, it->second.first, o.layout, s, seg_ptr);
-      o.layout.block_threads = it->second.second;
+      build_sgd_layout(K.ptr.p, K.tail.p, K.eps.p, n, (uint32_t)o.dim, it->second, false, o.layout, s, seg_ptr);
       return;
     }
   }
   const uint32_t chunks[] = {32, 64, 128, 256};
-  const uint32_t blocks[] = {128, 256};
   const uint32_t mid = (uint32_t)std::max<uint64_t>(1, o.total_epochs / 2);
   DevBuf<float> scratch(2 * n * o.dim, s);
   d2d(scratch.p, o.emb2.p, n * o.dim, s);
@@ -753,34 +750,30 @@ void tune_layout(umap_optimizer& o, const KeptEdges& K) {
   UB_CUDA(cudaEventCreate(&e0));
   UB_CUDA(cudaEventCreate(&e1));
   float best = 1e30f;
-  uint32_t best_chunk = 0, best_bt = 256;
+  uint32_t best_chunk = 0;
   for (uint32_t ch : chunks) {
     SgdLayout L;
-    build_sgd_layout(K.ptr.p, K.tail.p, K.eps.p, n, ch, L, s, seg_ptr);
-    for (uint32_t bt : blocks) {
-      L.block_threads = bt;
-      sgd_epoch(L, scratch.p, scratch.p + n * o.dim, p, mid, 0.5f, s);  // warm-up
-      UB_CUDA(cudaEventRecord(e0, s));
-      for (int r = 0; r < 2; ++r) sgd_epoch(L, scratch.p, scratch.p + n * o.dim, p, mid + r, 0.5f, s);
-      UB_CUDA(cudaEventRecord(e1, s));
-      UB_CUDA(cudaEventSynchronize(e1));
-      float ms = 0;
-      UB_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-      if (ms < best) {
-        best = ms;
-        best_chunk = ch;
-        best_bt = bt;
-      }
+    build_sgd_layout(K.ptr.p, K.tail.p, K.eps.p, n, (uint32_t)o.dim, ch, false, L, s, seg_ptr);
+    sgd_epoch(L, scratch.p, scratch.p + n * o.dim, p, mid, 0.5f, false, s);  // warm-up
+    UB_CUDA(cudaEventRecord(e0, s));
+    for (int r = 0; r < 2; ++r) sgd_epoch(L, scratch.p, scratch.p + n * o.dim, p, mid + r, 0.5f, r > 0, s);
+    UB_CUDA(cudaEventRecord(e1, s));
+    UB_CUDA(cudaEventSynchronize(e1));
+    float ms = 0;
+    UB_CUDA(cudaEventElapsedTime(&ms, e0, e1));
+    if (ms < best) {
+      best = ms;
+      best_chunk = ch;
+      o.layout = std::move(L);
     }
+    if (o.layout.max_degree <= ch) break;  // longer tasks would be the same whole rows
   }
   (void)cudaEventDestroy(e0);
   (void)cudaEventDestroy(e1);
-  build_sgd_layout(K.ptr.p, K.tail.p, K.eps.p, n, best_chunk, o.layout, s, seg_ptr);
-  o.layout.block_threads = best_bt;
   if (getenv("UMAP_B200_LOG"))
-    fprintf(stderr, "[umap_b200] autotune: chunk=%u block=%u (%.3f ms / 2 epochs)\n", best_chunk, best_bt, best);
+    fprintf(stderr, "[umap_b200] autotune: chunk=%u (%.3f ms / 2 epochs)\n", best_chunk, best);
   std::lock_guard<std::mutex> lock(g_tune_mu);
-  g_tuned[key] = {best_chunk, best_bt};
+  g_tuned[key] = best_chunk;
 }
 
 // ------------------------------------------------------------------ batched instances
@@ -886,7 +879,7 @@ std::unique_ptr<umap_optimizer> batch_new_impl(const umap_config& c, uint64_t n_
       const char* e = getenv("UMAP_B200_AUTOTUNE");
       return e && e[0] == '0';
     }();
-    if (no_tune || total_epochs < 2) build_sgd_layout(K.ptr.p, K.tail.p, K.eps.p, N, 0, o->layout, s, &so);
+    if (no_tune || total_epochs < 2) build_sgd_layout(K.ptr.p, K.tail.p, K.eps.p, N, (uint32_t)dims, 0, false, o->layout, s, &so);
     else tune_layout(*o, K);
   }
   set_l2_window(*o, true);
@@ -1080,7 +1073,7 @@ void finish_loaded_optimizer(umap_optimizer& o, const DevBuf<uint32_t>& head, co
   DevBuf<uint64_t> ptr(n + 1, s);
   segment_starts(head.p, E, n, ptr.p, s);
   const bool generic = o.metric_type == UMAP_METRIC_GENERIC;
-  build_sgd_layout(ptr.p, tail.p, eps.p, n, generic ? pick_chunk_generic(E) : 0, o.layout, s, nullptr, !generic);
+  build_sgd_layout(ptr.p, tail.p, eps.p, n, (uint32_t)o.dim, 0, generic, o.layout, s);
   set_l2_window(o, true);
   UB_CUDA(cudaStreamSynchronize(s));
 }
@@ -2230,7 +2223,7 @@ int umap_optimizer_tuning(const umap_optimizer* opt, uint32_t* chunk, uint32_t* 
   API_BEGIN
   need(opt, "optimizer");
   if (chunk) *chunk = opt->layout.chunk;
-  if (block_threads) *block_threads = opt->layout.block_threads;
+  if (block_threads) *block_threads = epoch_block_threads(opt->layout);
   API_END
 }
 
@@ -2238,8 +2231,11 @@ int umap_optimizer_layout_flags(const umap_optimizer* opt, uint32_t* flags) {
   API_BEGIN
   need(opt, "optimizer"); need(flags, "flags");
   *flags = (opt->layout.lane_major ? UMAP_LAYOUT_LANE_MAJOR : 0u) |
-           (opt->layout.short_epoch && !opt->layout.dram_epoch ? UMAP_LAYOUT_EIGHT_NEGATIVES : 0u) |
-           (opt->layout.dram_epoch ? UMAP_LAYOUT_TWELVE_NEGATIVES : 0u) |
+           (opt->layout.kernel == EpochKernel::Dram ? UMAP_LAYOUT_DRAM | UMAP_LAYOUT_TWELVE_NEGATIVES : 0u) |
+           (opt->layout.kernel == EpochKernel::Pool ? UMAP_LAYOUT_POOLED : 0u) |
+           (opt->layout.kernel == EpochKernel::Group4 ? UMAP_LAYOUT_GROUP_4 : 0u) |
+           (opt->layout.kernel == EpochKernel::Group8 ? UMAP_LAYOUT_GROUP_8 : 0u) |
+           (opt->layout.kernel == EpochKernel::Columns ? UMAP_LAYOUT_COLUMNS : 0u) |
            (opt->layout.order.p ? UMAP_LAYOUT_RENAMED : 0u) |
            (opt->metric_type == UMAP_METRIC_GENERIC ? UMAP_LAYOUT_GENERIC_RULE : 0u) |
            (opt->layout.task_order == TaskOrder::LengthRate ? UMAP_LAYOUT_RATE_ORDER : 0u) |

@@ -2,13 +2,11 @@
 // (K7).
 //
 // Layout.  The kept edges of the symmetric graph are grouped by head row and cut into tasks
-// of at most `chunk` edges (see SgdLayout).  A warp owns a slice of 32 tasks and a lane owns
-// one task, keeping the head row's live embedding in registers.  A slice's entries are lane
-// major when the embedding the epoch touches stays in L2: task l's entries are contiguous at
-// base + l * width (width = the slice's longest task rounded up to 4 entries, padding never
-// fires), so a lane's 4-entry window is one aligned 32-byte sector whatever the other lanes'
-// progress.  Otherwise (DRAM-bound sizes) entry e of task l sits at base + 32 e + l, so a
-// warp's loads cover whole 256-byte rows (see pick_lane_major).  The reference writes a
+// of at most `chunk` edges (see SgdLayout), packed 32 to a slice; the head row's live embedding
+// is kept in registers while its task runs.  A slice's entries are lane major: task l's entries
+// are contiguous at base + l * width (width = the slice's longest task rounded up to 4 entries,
+// padding never fires).  In DRAM-bound layouts entry e of task l sits at base + 32 e + l instead,
+// so a warp's loads cover whole 256-byte rows (see pick_epoch_kernel).  The reference writes a
 // head row only from edges whose head it is (optimize_layout_euclidean.rs:281-306, :338),
 // so a task that is a whole row reproduces the reference's sequential per-row order with
 // no lost head updates; the rare long rows (kNN hubs) are split so that one row cannot
@@ -28,32 +26,27 @@
 #include <cstdint>
 #include <cstdlib>
 #include <cstring>
+#include <utility>
 #include <vector>
 
 #include "ub_internal.hpp"
+#include "umma.cuh"
 
 namespace ub {
 namespace {
 
 constexpr uint32_t PAD_ROW = 0xFFFFFFFFu;
 
-// The epoch kernel comes in two register budgets.  Large graphs (many waves of warps) are
-// bound by instruction issue and L2 sector throughput: 4 negative rows fetched together and
-// 5 resident 256-thread blocks per SM (48 registers).  Graphs that fill about two waves or
-// fewer are bound by the chain of dependent loads of their busiest lanes: 8 negative rows
-// fetched together (one round trip for a firing's usual 4-6 negatives) and 4 blocks per SM.
-// On the 2M-point workload (500 epochs, SGD ms) the wide budget's occupancy beats the extra
-// round trip of a firing's fifth negative: 4 / 5: 314.0, 8 / 4: 317.6, 6 / 4: 330.9, 4 / 4:
-// 343.5, 5 / 4: 349.9 (5 and 6 rows at 5 blocks per SM spill more than 4 / 5's 16 bytes).
-constexpr int NB_WIDE = 4, MINB_WIDE = 5;
-constexpr int NB_SHORT = 8, MINB_SHORT = 4;
-// Renamed DRAM-bound layouts: 12 negative rows fetched together, 3 blocks per SM.  Their random
-// row loads go to DRAM and their warps are limited by registers either way, so more loads in
-// flight per lane beat more warps (30 epochs of a 20M-point roll: 8 / 4: 310.8 ms, 10 / 3:
+// DRAM-bound layouts (sgd_epoch_dram): 12 negative rows fetched together, 3 blocks per SM.  Their
+// random row loads go to DRAM and their warps are limited by registers either way, so more loads
+// in flight per lane beat more warps (30 epochs of a 20M-point roll: 8 / 4: 310.8 ms, 10 / 3:
 // 295.1, 12 / 3: 295.2, 12 / 2: 313.4, 16 / 2: 316.0, 24 / 2: 317.7; 40M points, 24 epochs:
-// 8 / 4: 590.4, 12 / 3: 562.6, 16 / 2: 564.9).  Small latency-bound graphs keep 8 / 4: with
-// 12 / 3 the warm start's 100k-point subsample fit took 38.4-38.9 ms against 30.5-31.6 ms.
+// 8 / 4: 590.4, 12 / 3: 562.6, 16 / 2: 564.9).
 constexpr int NB_DRAM = 12, MINB_DRAM = 3;
+// The pooled kernel: 8 negative rows fetched together, 8 blocks of 128 threads per SM (64
+// registers).  2M points, us per epoch: 8 / 8: 482, 6 / 8: 480, 6 / 9: 481, 4 / 10: 516, 4 / 8: 511;
+// 300k points: 92, 98, 98, 106, 106.
+constexpr int POOL_BT = 128, NB_POOL = 8, MINB_POOL = 8;
 
 // ------------------------------------------------------------------------------ negatives' RNG
 // Counter-based: the firing of entry `idx` at `epoch` draws its negatives in pairs; pair t is
@@ -109,37 +102,22 @@ __device__ __forceinline__ bool fires_at(uint32_t n, uint32_t q) {
 }
 // Negatives drawn by the firing at epoch n (n * neg < 2^32 is checked on the host):
 // y(n) - y(p) with y(x) = fires_by(x * neg) and p the epoch of the previous firing, or
-// y(n) - 1 for the first.  Firings are floor(2^32 / Q) or one more epochs apart, so p is found
-// among a few candidates below n - floor(2^32 / Q) + 1 with the cheap test above (the float
-// estimate of the gap is within one epoch: a second firing needs n >= 2 * 2^32 / Q and epochs
-// stay below MAX_EPOCHS = 2^21, checked on the host; fire_epoch is the exact fallback).
-// A two-candidate form with an exact integer gap (one fewer fires_at test, no fallback)
-// measured 1.7% slower on the 2M workload (317.6 against 312.3 ms per 500 epochs).
+// y(n) - 1 for the first.  With n Q = m 2^32 + f (0 <= f < Q, as it fires at n) the previous firing
+// is t = floor((2^32 + f) / Q) epochs back and p Q = (m - 1) 2^32 + g, g = (2^32 + f) - t Q, so
+// y(n) = m neg + floor(neg f / 2^32) and y(p) = (m - 1) neg + floor(neg g / 2^32).  t <= n <
+// MAX_EPOCHS = 2^21 (checked on the host), so the float quotient is within one of it and g's sign
+// and size correct it.
 __device__ __forceinline__ uint32_t negatives_at(uint32_t n, uint32_t q, uint32_t neg) {
-  const int64_t y = (int64_t)fires_by(n * neg, q);
-  const uint64_t m = fires_by(n, q);
-  int64_t prev = 1;
-  if (m > 1) {
-    const int64_t g0 = (int64_t)__fdividef(4294967296.0f, (float)q + 1.0f);
-    uint32_t pe = 0;
-#pragma unroll
-    for (int t = 1; t >= -2; --t) {
-      const int64_t x = (int64_t)n - g0 + t;
-      if (pe == 0 && x >= 1 && x < (int64_t)n && fires_at((uint32_t)x, q)) pe = (uint32_t)x;
-    }
-    if (pe == 0) pe = fire_epoch(m - 1, q);
-    prev = (int64_t)fires_by(pe * neg, q);
-  }
-  const int64_t d = y - prev;
+  const uint64_t nq = (uint64_t)n * q + n, Q = (uint64_t)q + 1;
+  const uint32_t f = (uint32_t)nq, m = (uint32_t)(nq >> 32);
+  const int64_t span = (int64_t)(((uint64_t)1 << 32) + f);
+  const uint32_t t = (uint32_t)__fdividef(4294967296.0f + (float)f, (float)Q);
+  int64_t g = span - (int64_t)((uint64_t)t * Q);
+  if (g < 0) g += (int64_t)Q;
+  else if (g >= (int64_t)Q) g -= (int64_t)Q;
+  const uint32_t upto = __umulhi(neg, f);
+  const int32_t d = (int32_t)(neg + upto - (m > 1 ? __umulhi(neg, (uint32_t)g) : 1u));
   return d > 0 ? (uint32_t)d : 0u;
-}
-
-// Rust f32::clamp(-4, 4) (utils/clip.rs:13-15): NaN passes through.
-__device__ __forceinline__ float clip4(float v) {
-  float x = v;
-  if (x < -4.0f) x = -4.0f;
-  if (x > 4.0f) x = 4.0f;
-  return x;
 }
 
 // Two-lane FP32 arithmetic on a 2-D row (each lane the same IEEE operation as the scalar one).
@@ -186,6 +164,21 @@ __device__ __forceinline__ void load_row(float (&v)[DIM], const float* p) {
     for (int d = 0; d < DIM; ++d) v[d] = p[d];
   }
 }
+// The same through L2 only.
+template <int DIM>
+__device__ __forceinline__ void load_row_l2(float (&v)[DIM], const float* p) {
+  if constexpr (DIM == 2) {
+    const float2 t = __ldcg(reinterpret_cast<const float2*>(p));
+    v[0] = t.x;
+    v[1] = t.y;
+  } else if constexpr (DIM == 4) {
+    const float4 t = __ldcg(reinterpret_cast<const float4*>(p));
+    v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+  } else {
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) v[d] = __ldcg(p + d);
+  }
+}
 template <int DIM>
 __device__ __forceinline__ void store_row(float* p, const float (&v)[DIM]) {
   if constexpr (DIM == 2) {
@@ -228,6 +221,64 @@ __device__ __forceinline__ float metric_coeff(float ds, float a, float two_b, fl
   return __fdividef(scale * (w + bias), *den);
 }
 
+// The Euclidean rule's step of a head row (optimize_layout_euclidean.rs:284-306, :319-339) with
+// the shortest chain from the row to its update, which is what a task's firings wait for: the
+// squared distance carries the smallest normal number along (a subnormal one would cost scaling
+// instructions around each approximate log2 / exp2 / reciprocal; the move at such a distance is
+// below 1e-16 either way), ds^b = 2^(b log2 ds), and the denominators are one fused step behind it.
+__device__ __forceinline__ float ftz_log2(float x) { float r; asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
+__device__ __forceinline__ float ftz_exp2(float x) { float r; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
+__device__ __forceinline__ float ftz_rcp(float x) { float r; asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
+// Rust f32::clamp(-4, 4) (utils/clip.rs:13-15): NaN passes through.
+__device__ __forceinline__ float clip4(float v) {
+  float r;
+  asm("min.NaN.f32 %0, %1, 0f40800000;" : "=f"(r) : "f"(v));
+  asm("max.NaN.f32 %0, %1, 0fC0800000;" : "=f"(r) : "f"(r));
+  return r;
+}
+template <int DIM>
+__device__ __forceinline__ float square_ftz(const float (&df)[DIM]) {
+  float ds = 1.17549435e-38f;
+#pragma unroll
+  for (int d = 0; d < DIM; ++d) ds = fmaf(df[d], df[d], ds);
+  return ds;
+}
+// Attraction coefficient -2ab ds^b / (ds (a ds^b ds + 1)) as num * inv.
+__device__ __forceinline__ void attract_terms(float ds, const SgdParams& p, float& num, float& inv) {
+  const float pb = ftz_exp2(p.b * ftz_log2(ds));
+  num = p.neg_attr * pb;
+  inv = ftz_rcp(fmaf(p.a * ds * ds, pb, ds));
+}
+// 1 / ((0.001 + ds)(a ds^b ds + 1)), the repulsion coefficient over 2 gamma b.
+__device__ __forceinline__ float repel_inv(float ds, const SgdParams& p) {
+  const float u = 0.001f + ds, v = u * (p.a * ds);
+  return ftz_rcp(fmaf(v, ftz_exp2(p.b * ftz_log2(ds)), u));
+}
+// Attractive move g of the head row (the tail gets -g).
+template <int DIM>
+__device__ __forceinline__ void attract(float (&cur)[DIM], const float (&o)[DIM], float (&g)[DIM], const SgdParams& p,
+                                        float alpha) {
+  float df[DIM], num, inv;
+#pragma unroll
+  for (int d = 0; d < DIM; ++d) df[d] = cur[d] - o[d];
+  attract_terms(square_ftz<DIM>(df), p, num, inv);
+#pragma unroll
+  for (int d = 0; d < DIM; ++d) g[d] = clip4((num * df[d]) * inv) * alpha;
+}
+// Repulsive move from row o, where `apply`; a NaN distance (a NaN row) moves nothing.
+template <int DIM>
+__device__ __forceinline__ void repel(float (&cur)[DIM], const float (&o)[DIM], bool apply, const SgdParams& p,
+                                      float alpha) {
+  float df[DIM];
+#pragma unroll
+  for (int d = 0; d < DIM; ++d) df[d] = cur[d] - o[d];
+  const float ds = square_ftz<DIM>(df), inv = repel_inv(ds, p);
+  if (apply && ds > 0.0f) {
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) cur[d] = fmaf(clip4((p.pos_rep * df[d]) * inv), alpha, cur[d]);
+  }
+}
+
 // One fired edge (optimize_layout_euclidean.rs:278-343, or with GEN the generic-metric rule
 // of optimize_layout_generic.rs:57-121): attractive step on (head, tail), then `nneg`
 // negative samples, all reading the snapshot buffer.  The tail row and a batch of negative
@@ -235,15 +286,14 @@ __device__ __forceinline__ float metric_coeff(float ds, float a, float two_b, fl
 template <int DIM, bool GEN, int NEG_BATCH>
 __device__ __forceinline__ void fired_edge(float (&cur)[DIM], uint32_t r, uint32_t k, uint32_t nneg,
                                            float* snap, const SgdParams& p, float alpha, uint64_t idx,
-                                           uint32_t epoch, uint64_t seed, uint32_t seg_lo, uint32_t seg_n) {
-  const float a = p.a, b = p.b;
+                                           uint32_t epoch, uint32_t seg_lo, uint32_t seg_n) {
   float* oth = snap + (uint64_t)k * DIM;
   float o[DIM];
   load_row<DIM>(o, oth);
   // Negative q uses half (q & 1) of pair (q >> 1) for this (entry, epoch).
   uint32_t kk[NEG_BATCH];
   float ob[NEG_BATCH][DIM];
-  const NegRng rng(seed, idx, epoch);
+  const NegRng rng(p.seed, idx, epoch);
   uint64_t rnd = 0;
   uint32_t rpair = 0xFFFFFFFFu;
   auto fetch = [&](uint32_t q0) {
@@ -272,31 +322,20 @@ __device__ __forceinline__ void fired_edge(float (&cur)[DIM], uint32_t r, uint32
   };
   fetch(0);
   // attractive step (:284-306)
-  float ds = 0.0f;
-#pragma unroll
-  for (int d = 0; d < DIM; ++d) { const float df = cur[d] - o[d]; ds += df * df; }
   float g[DIM];
   if constexpr (GEN) {
     // head += clip(c * grad) alpha; tail += clip(c * rev_grad) alpha with rev_grad = -grad
-    float den;
-    const float gc = metric_coeff(ds, a, p.two_b, p.two_b, -1.0f, &den);
+    float ds = 0.0f, den;
 #pragma unroll
-    for (int d = 0; d < DIM; ++d) {
-      g[d] = clip4(gc * __fdividef(cur[d] - o[d], den)) * alpha;
-      cur[d] += g[d];
-    }
+    for (int d = 0; d < DIM; ++d) { const float df = cur[d] - o[d]; ds += df * df; }
+    const float gc = metric_coeff(ds, p.a, p.two_b, p.two_b, -1.0f, &den);
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) g[d] = clip4(gc * __fdividef(cur[d] - o[d], den)) * alpha;
   } else {
-    float gc = 0.0f;
-    if (ds > 0.0f) {
-      const float pb = __powf(ds, b);
-      gc = __fdividef(p.neg_attr * pb, ds * (a * pb * ds + 1.0f));
-    }
-#pragma unroll
-    for (int d = 0; d < DIM; ++d) {
-      g[d] = clip4(gc * (cur[d] - o[d])) * alpha;
-      cur[d] += g[d];
-    }
+    attract<DIM>(cur, o, g, p, alpha);
   }
+#pragma unroll
+  for (int d = 0; d < DIM; ++d) cur[d] += g[d];
   sub_row<DIM>(oth, g);
   // negative samples (:313-341)
   for (uint32_t q0 = 0; q0 < nneg; q0 += NEG_BATCH) {
@@ -305,124 +344,68 @@ __device__ __forceinline__ void fired_edge(float (&cur)[DIM], uint32_t r, uint32
     for (int q = 0; q < NEG_BATCH; ++q) {
       if (q0 + q >= nneg) break;
       if (kk[q] == r) continue;
-      if constexpr (DIM == 2 && !GEN) {
-        // the same operations as the generic-DIM code below, two columns per instruction
-        const uint64_t c2 = pk2(cur[0], cur[1]);
-        const uint64_t df2 = sub2(c2, pk2(ob[q][0], ob[q][1]));
-        float df0, df1;
-        up2(df2, df0, df1);
-        const float dsn = df0 * df0 + df1 * df1;
-        float gr = 0.0f;
-        if (dsn > 0.0f) {
-          const float pb = __powf(dsn, b);
-          gr = __fdividef(p.pos_rep, (0.001f + dsn) * (a * pb * dsn + 1.0f));
-        }
-        if (gr > 0.0f) {
-          float t0, t1;
-          up2(mul2(pk2(gr, gr), df2), t0, t1);
-          up2(fma2(pk2(clip4(t0), clip4(t1)), pk2(alpha, alpha), c2), cur[0], cur[1]);
-        }
-        continue;
-      }
-      float dsn = 0.0f;
-#pragma unroll
-      for (int d = 0; d < DIM; ++d) { const float df = cur[d] - ob[q][d]; dsn += df * df; }
       if constexpr (GEN) {
-        float den;
-        const float gr = metric_coeff(dsn, a, p.two_b, p.pos_rep, 0.0f, &den);
+        float dsn = 0.0f, den;
+#pragma unroll
+        for (int d = 0; d < DIM; ++d) { const float df = cur[d] - ob[q][d]; dsn += df * df; }
+        const float gr = metric_coeff(dsn, p.a, p.two_b, p.pos_rep, 0.0f, &den);
 #pragma unroll
         for (int d = 0; d < DIM; ++d) cur[d] += clip4(gr * __fdividef(cur[d] - ob[q][d], den)) * alpha;
       } else {
-        float gr = 0.0f;
-        if (dsn > 0.0f) {
-          const float pb = __powf(dsn, b);
-          gr = __fdividef(p.pos_rep, (0.001f + dsn) * (a * pb * dsn + 1.0f));
-        }
-        if (gr > 0.0f) {
-#pragma unroll
-          for (int d = 0; d < DIM; ++d) cur[d] += clip4(gr * (cur[d] - ob[q][d])) * alpha;
-        }
+        repel<DIM>(cur, ob[q], true, p, alpha);
       }
     }
   }
 }
 
-// Variant with independent lane progress: each lane walks its own task through a small
-// register window of entries (refilled on demand, W loads in flight), so a warp runs as long
-// as its busiest task rather than its busiest lane of every batch.
-#ifndef UB_SGD2_W
-#define UB_SGD2_W 4
-#endif
-template <int DIM, bool GEN, int NEG_BATCH, int MINB, bool LM>
-__global__ void __launch_bounds__(256, MINB) sgd_epoch_kernel2(
+// DRAM-bound layouts (1-D and 2-D, interleaved entries): a lane per task with independent progress -
+// each lane finds the firings of 16 of its entries at a time and walks them - so a warp runs as
+// long as its busiest task.  (A 4-entry window held in registers, refilled about once per firing,
+// took 5M-point epochs from 1,156 to 1,530 us.)
+constexpr int DRAM_WIN = 16;
+template <int DIM>
+__global__ void __launch_bounds__(256, MINB_DRAM) sgd_epoch_dram(
     const uint64_t* __restrict__ slice_base, const uint32_t* __restrict__ slice_width,
     const uint32_t* __restrict__ split_mask, const uint32_t* __restrict__ rowid,
     const uint2* __restrict__ entry, uint64_t n_slices, float* __restrict__ live, float* snap,
     SgdParams p, uint32_t epoch, float alpha) {
-  constexpr int W = UB_SGD2_W;
   const uint64_t slice = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint32_t lane = threadIdx.x & 31;
   if (slice >= n_slices) return;
   const uint32_t r = rowid[slice * 32 + lane];
   const bool active = r != PAD_ROW;
   const uint32_t width = active ? slice_width[slice] : 0u;
-  const uint64_t base = slice_base[slice];
+  const uint64_t first = slice_base[slice] + lane;
   const bool split = (split_mask[slice] >> lane) & 1u;
-  uint32_t seg_lo = 0, seg_n = p.n_vertices;
-  if (p.row_seg && active) {
-    const uint32_t sg = p.row_seg[r];
-    seg_lo = (uint32_t)p.seg_off[sg];
-    seg_n = (uint32_t)(p.seg_off[sg + 1] - p.seg_off[sg]);
-  }
   float cur[DIM], start[DIM];
   float* hrow = live + (uint64_t)(active ? r : 0) * DIM;
-  if (active) load_row<DIM>(cur, hrow);
-  else
-#pragma unroll
-    for (int d = 0; d < DIM; ++d) cur[d] = 0.0f;
+  load_row<DIM>(cur, hrow);
 #pragma unroll
   for (int d = 0; d < DIM; ++d) start[d] = cur[d];
-  const uint32_t n = epoch;
-  const uint64_t seed = p.seed;
-  static_assert(W % 4 == 0, "windows are whole 4-entry sectors");
-  // this lane's entries: contiguous (lane major) or every 32nd (interleaved)
-  const uint2* lent = LM ? entry + base + (uint64_t)lane * width : entry + base + lane;
-  uint2 win[W];
+  const uint2* lent = entry + first;
   uint32_t mask = 0, ew = 0, ebase = 0;
+  uint2 nx = make_uint2(0u, 0u);  // the next fired entry
   for (;;) {
-    while (mask == 0 && ew < width) {
-      ebase = ew;
-      if (LM) {
-        // width is a multiple of W (slice_meta_kernel): the window lies inside the lane's entries
+    if (mask == 0) {
+      while (mask == 0 && ew < width) {
+        ebase = ew;
 #pragma unroll
-        for (int j = 0; j < W; j += 2) {
-          const uint4 v = __ldg(reinterpret_cast<const uint4*>(lent + ew + j));
-          win[j] = make_uint2(v.x, v.y);
-          win[j + 1] = make_uint2(v.z, v.w);
+        for (int j = 0; j < DRAM_WIN; ++j) {
+          const uint32_t q = ew + j < width ? __ldg(&lent[(uint64_t)(ew + j) * 32].y) : 0u;
+          mask |= fires_at(epoch, q) ? 1u << j : 0u;
         }
-      } else {
-#pragma unroll
-        for (int j = 0; j < W; ++j) {
-          const uint32_t e = ew + j;
-          win[j] = e < width ? __ldg(lent + (uint64_t)e * 32) : make_uint2(0u, 0u);
-        }
+        ew += DRAM_WIN;
       }
-#pragma unroll
-      for (int j = 0; j < W; ++j)
-        if (fires_at(n, win[j].y)) mask |= 1u << j;
-      ew += W;
+      if (mask) nx = __ldg(lent + (uint64_t)(ebase + __ffs(mask) - 1) * 32);
     }
     if (!__any_sync(0xFFFFFFFFu, mask != 0)) break;
     if (mask) {
-      const int j = __ffs(mask) - 1;
+      const uint2 en = nx;
+      const uint64_t idx = first + (uint64_t)(ebase + __ffs(mask) - 1) * 32;
       mask &= mask - 1;
-      uint2 en = win[0];
-#pragma unroll
-      for (int t = 1; t < W; ++t)
-        if (t == j) en = win[t];
-      const uint32_t nneg = negatives_at(n, en.y, p.neg_rate);
-      const uint64_t idx = LM ? base + (uint64_t)lane * width + ebase + j : base + (uint64_t)(ebase + j) * 32 + lane;
-      fired_edge<DIM, GEN, NEG_BATCH>(cur, r, en.x, nneg, snap, p, alpha, idx, epoch, seed, seg_lo, seg_n);
+      if (mask) nx = __ldg(lent + (uint64_t)(ebase + __ffs(mask) - 1) * 32);
+      fired_edge<DIM, false, NB_DRAM>(cur, r, en.x, negatives_at(epoch, en.y, p.neg_rate), snap, p, alpha, idx, epoch,
+                                      0u, p.n_vertices);
     }
   }
   if (active) {
@@ -435,7 +418,152 @@ __global__ void __launch_bounds__(256, MINB) sgd_epoch_kernel2(
   }
 }
 
-// Any dimension (n_components > 4): same algorithm, head row in global memory (owned by this
+// A firing's rows as the grouped kernels fetch them: slots 0..6 are its first seven negatives, slot 7
+// its tail.  At the default negative_sample_rate of 5 most firings draw 4 to 7 negatives (up to 10
+// where an edge that fires almost every epoch skips one; those past the slots are read one by one.
+// 16 slots measured 5% slower).
+constexpr int SLOTS = 8, NEG_SLOTS = SLOTS - 1, TAIL_SLOT = SLOTS - 1;
+
+// Negative q of the firing whose generator is `rng`.
+__device__ __forceinline__ uint32_t negative_row(const NegRng& rng, uint32_t q, uint32_t seg_lo, uint32_t seg_n) {
+  const uint64_t rnd = rng.pair(q >> 1);
+  return seg_lo + __umulhi((q & 1) ? (uint32_t)(rnd >> 32) : (uint32_t)rnd, seg_n);
+}
+
+// The epoch of L2-resident layouts: a block of POOL_BT threads takes as many tasks.  For every
+// window of 32 entries it (1) evaluates the schedule of all its tasks' entries, 8 lanes reading 64
+// consecutive bytes of a task, which leaves one bit per entry, (2) sorts the tasks that fire by
+// their number of firings (counting sort, descending), and (3) gives thread i the i-th of them.
+// What bounds it: the random rows - per firing a tail, its atomic add and about 5 negatives, one
+// 32-byte L2 sector each.  Such a mix runs at most at 260 G/s here whatever the path (plain,
+// L2-only, asynchronous copies), 0.385 ms of the 2M-point epoch.  A warp whose lanes own fixed tasks
+// has half of them idle (its tasks' firings differ from epoch to epoch), and reading the schedule in
+// per-lane windows cost a quarter more requests: 2M points 537 -> 474 us per epoch, 300k 102 -> 92,
+// 70k 39 -> 34.  Larger pools (256 or 512 tasks, warps taking 32 at a time from the sorted list)
+// were slower: a block's heavy warps outlast the others, 727 / 945 us at 2M.
+// `early` lets the next epoch's blocks start as soon as this launch's last ones have, otherwise at
+// its end (see sgd_epoch).
+constexpr int POOL_WIN = 32;
+template <int DIM, bool GEN>
+__global__ void __launch_bounds__(POOL_BT, MINB_POOL) sgd_epoch_pool(
+    const uint64_t* __restrict__ slice_base, const uint32_t* __restrict__ slice_width,
+    const uint32_t* __restrict__ split_mask, const uint32_t* __restrict__ rowid,
+    const uint2* __restrict__ entry, uint64_t n_slices, float* __restrict__ live, float* snap,
+    SgdParams p, uint32_t epoch, float alpha, bool early) {
+  constexpr int SL = POOL_BT / 32;  // slices: one per warp while the schedule is evaluated
+  __shared__ uint32_t s_mask[POOL_BT];
+  __shared__ uint8_t s_order[POOL_BT];
+  __shared__ uint64_t s_base[SL];
+  __shared__ uint32_t s_width[SL], s_split[SL], s_hist[POOL_WIN + 1], s_total;
+  const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint64_t slice0 = (uint64_t)blockIdx.x * SL;
+  if (early) umma::grid_release();
+  if (tid < SL) {
+    const bool in = slice0 + tid < n_slices;
+    s_base[tid] = in ? slice_base[slice0 + tid] : 0;
+    s_width[tid] = in ? slice_width[slice0 + tid] : 0;
+    s_split[tid] = in ? split_mask[slice0 + tid] : 0;
+  }
+  __syncthreads();
+  uint32_t width = 0;  // the block's longest task
+#pragma unroll
+  for (int w = 0; w < SL; ++w) width = max(width, s_width[w]);
+  for (uint32_t ew = 0; ew < width; ew += POOL_WIN) {
+    if (tid <= POOL_WIN) s_hist[tid] = 0;
+    {
+      const uint32_t sub = lane >> 3, el = lane & 7, wd = s_width[warp];
+      const uint32_t lim = ew < wd ? min(wd - ew, (uint32_t)POOL_WIN) : 0u;
+      const uint2* src = entry + s_base[warp] + ew + el;
+#pragma unroll 1
+      for (uint32_t t = 0; t < 32; t += 16) {
+        uint32_t m[4] = {0, 0, 0, 0};
+#pragma unroll
+        for (uint32_t h = 0; h < POOL_WIN; h += 16) {
+          if (h >= lim) break;  // the same for the whole warp
+          uint32_t q[8];        // 8 loads in flight before the first vote
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const uint32_t j = h + (i & 1) * 8, tt = t + (i >> 1) * 4 + sub;
+            q[i] = j + el < lim ? __ldg(&src[(uint64_t)tt * wd + j].y) : 0u;
+          }
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const unsigned b = __ballot_sync(0xFFFFFFFFu, fires_at(epoch, q[i]));
+            m[i >> 1] |= ((b >> (8 * sub)) & 0xFFu) << (h + (i & 1) * 8);
+          }
+        }
+        if (el == 0) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) s_mask[warp * 32 + t + i * 4 + sub] = m[i];
+        }
+      }
+    }
+    __syncthreads();
+    const uint32_t c = __popc(s_mask[tid]);
+    const unsigned peers = __match_any_sync(0xFFFFFFFFu, c);
+    const int leader = __ffs(peers) - 1;
+    if ((int)lane == leader) atomicAdd(&s_hist[c], (uint32_t)__popc(peers));
+    __syncthreads();
+    if (warp == 0) {  // s_hist[k] = number of tasks with more than k firings (k >= 1)
+      const uint32_t k = 32 - lane, h = s_hist[k];
+      uint32_t v = h;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t u = __shfl_up_sync(0xFFFFFFFFu, v, o);
+        if ((int)lane >= o) v += u;
+      }
+      s_hist[k] = v - h;
+      if (lane == 31) s_total = v;
+    }
+    __syncthreads();
+    uint32_t pos = 0;
+    if ((int)lane == leader && c) pos = atomicAdd(&s_hist[c], (uint32_t)__popc(peers));
+    pos = __shfl_sync(0xFFFFFFFFu, pos, leader) + __popc(peers & ((1u << lane) - 1u));
+    if (c) s_order[pos] = (uint8_t)tid;
+    if (ew == 0) umma::grid_wait();
+    __syncthreads();
+    if (tid < s_total) {
+      const uint32_t o = s_order[tid], sl = o >> 5, tl = o & 31;
+      const uint32_t row = rowid[(slice0 + sl) * 32 + tl];
+      const uint64_t first = s_base[sl] + (uint64_t)tl * s_width[sl] + ew;
+      const uint2* lent = entry + first;
+      uint32_t m = s_mask[o], e = (uint32_t)__ffs(m) - 1;
+      uint32_t seg_lo = 0, seg_n = p.n_vertices;
+      if (p.row_seg) {
+        const uint32_t sg = p.row_seg[row];
+        seg_lo = (uint32_t)p.seg_off[sg];
+        seg_n = (uint32_t)(p.seg_off[sg + 1] - p.seg_off[sg]);
+      }
+      uint2 nx = __ldg(lent + e);
+      float cur[DIM], start[DIM];
+      float* hrow = live + (uint64_t)row * DIM;
+      load_row<DIM>(cur, hrow);
+#pragma unroll
+      for (int d = 0; d < DIM; ++d) start[d] = cur[d];
+      while (m) {
+        const uint2 en = nx;
+        const uint64_t idx = first + e;
+        m &= m - 1;
+        if (m) {
+          e = (uint32_t)__ffs(m) - 1;
+          nx = __ldg(lent + e);
+        }
+        fired_edge<DIM, GEN, NB_POOL>(cur, row, en.x, negatives_at(epoch, en.y, p.neg_rate), snap, p, alpha, idx, epoch,
+                                      seg_lo, seg_n);
+      }
+      if ((s_split[sl] >> tl) & 1u) {
+#pragma unroll
+        for (int d = 0; d < DIM; ++d) atomicAdd(hrow + d, cur[d] - start[d]);
+      } else {
+        store_row<DIM>(hrow, cur);
+      }
+    }
+    __syncthreads();
+  }
+  if (!early) umma::grid_release();
+}
+
+// More than 128 columns: same algorithm, a thread per task, head row in global memory (owned by this
 // lane for whole-row tasks; split tasks accumulate their delta in place with atomics).  GEN
 // selects the generic-metric rule as in fired_edge.
 template <bool GEN>
@@ -443,7 +571,7 @@ __global__ void __launch_bounds__(256) sgd_epoch_anydim(
     const uint64_t* __restrict__ slice_base, const uint32_t* __restrict__ slice_width,
     const uint32_t* __restrict__ split_mask, const uint32_t* __restrict__ rowid,
     const uint2* __restrict__ entry, uint64_t n_slices, float* __restrict__ live, float* snap,
-    SgdParams p, uint32_t epoch, float alpha, bool lane_major) {
+    SgdParams p, uint32_t epoch, float alpha) {
   const uint64_t slice = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint32_t lane = threadIdx.x & 31;
   if (slice >= n_slices) return;
@@ -462,13 +590,13 @@ __global__ void __launch_bounds__(256) sgd_epoch_anydim(
   float* cur = live + (uint64_t)r * dim;
   const uint32_t n = epoch;
   const uint64_t seed = p.seed;
-  const float a = p.a, b = p.b;
+  const float a = p.a;
   auto add = [&](uint32_t d, float v) {
     if (split) atomicAdd(cur + d, v);
     else cur[d] += v;
   };
   for (uint32_t e = 0; e < width; ++e) {
-    const uint64_t idx = lane_major ? base + (uint64_t)lane * width + e : base + (uint64_t)e * 32 + lane;
+    const uint64_t idx = base + (uint64_t)lane * width + e;
     const uint2 en = __ldcs(entry + idx);
     if (!fires_at(n, en.y)) continue;
     float* oth = snap + (uint64_t)en.x * dim;
@@ -477,9 +605,10 @@ __global__ void __launch_bounds__(256) sgd_epoch_anydim(
     float gc = 0.0f, den = 1.0f;
     if constexpr (GEN) {
       gc = metric_coeff(ds, a, p.two_b, p.two_b, -1.0f, &den);
-    } else if (ds > 0.0f) {
-      const float pb = __powf(ds, b);
-      gc = __fdividef(p.neg_attr * pb, ds * (a * pb * ds + 1.0f));
+    } else {
+      float num, inv;
+      attract_terms(ds + 1.17549435e-38f, p, num, inv);
+      gc = num * inv;
     }
     for (uint32_t d = 0; d < dim; ++d) {
       const float cd = cur[d], od = oth[d];
@@ -503,14 +632,366 @@ __global__ void __launch_bounds__(256) sgd_epoch_anydim(
         const float gr = metric_coeff(dsn, a, p.two_b, p.pos_rep, 0.0f, &dn);
         for (uint32_t d = 0; d < dim; ++d) add(d, clip4(gr * __fdividef(cur[d] - ob[d], dn)) * alpha);
       } else {
-        float gr = 0.0f;
-        if (dsn > 0.0f) {
-          const float pb = __powf(dsn, b);
-          gr = __fdividef(p.pos_rep, (0.001f + dsn) * (a * pb * dsn + 1.0f));
-        }
+        const float gr = p.pos_rep * repel_inv(dsn + 1.17549435e-38f, p);
         if (gr > 0.0f)
           for (uint32_t d = 0; d < dim; ++d) add(d, clip4(gr * (cur[d] - ob[d])) * alpha);
       }
+    }
+  }
+}
+
+// ------------------------------------------------------------------------------ grouped epochs
+// Entries whose schedule a group of G lanes evaluates together (one per lane and step).
+constexpr int group_window(int g) { return g > 16 ? g : 16; }
+
+
+// What a lane knows of its group's task, and the group's current window of entries.
+template <int G>
+struct GroupTask {
+  uint32_t gl, gshift, lt, tl, r, width, seg_lo, seg_n;
+  uint64_t base;
+  bool active, split;
+
+  __device__ __forceinline__ GroupTask(const uint64_t* slice_base, const uint32_t* slice_width,
+                                       const uint32_t* split_mask, const uint32_t* rowid, const SgdParams& p,
+                                       uint64_t slice, uint64_t task) {
+    const uint32_t lane = threadIdx.x & 31;
+    gl = lane & (G - 1);
+    gshift = lane & ~(uint32_t)(G - 1);
+    lt = threadIdx.x / G;
+    tl = (uint32_t)(task & 31);
+    r = rowid[task];
+    active = r != PAD_ROW;
+    width = slice_width[slice];
+    base = slice_base[slice];
+    split = (split_mask[slice] >> tl) & 1u;
+    seg_lo = 0;
+    seg_n = p.n_vertices;
+    if (p.row_seg && active) {
+      const uint32_t sg = p.row_seg[r];
+      seg_lo = (uint32_t)p.seg_off[sg];
+      seg_n = (uint32_t)(p.seg_off[sg + 1] - p.seg_off[sg]);
+    }
+  }
+  __device__ __forceinline__ uint64_t entry_index(uint32_t e) const { return base + (uint64_t)tl * width + e; }
+  // Fires of the window [ew, ew + group_window(G)): returns their mask and lists {tail, negatives} in
+  // `fire`, in entry order.
+  __device__ __forceinline__ uint32_t window(const uint2* __restrict__ entry, uint32_t ew,
+                                             uint32_t epoch, uint32_t neg_rate, uint2* fire) const {
+    constexpr int EPL = group_window(G) / G;
+    uint2 en[EPL];
+#pragma unroll
+    for (int i = 0; i < EPL; ++i) {
+      const uint32_t e = ew + i * G + gl;
+      en[i] = active && e < width ? __ldg(entry + entry_index(e)) : make_uint2(0u, 0u);
+    }
+    uint32_t m = 0;
+#pragma unroll
+    for (int i = 0; i < EPL; ++i) {
+      const bool f = fires_at(epoch, en[i].y);
+      const uint32_t b = (__ballot_sync(0xFFFFFFFFu, f) >> gshift) & (G == 32 ? 0xFFFFFFFFu : (1u << (G & 31)) - 1u);
+      if (f) fire[__popc(m) + __popc(b & ((1u << gl) - 1u))] = make_uint2(en[i].x, negatives_at(epoch, en[i].y, neg_rate));
+      m |= b << (i * G);
+    }
+    return m;
+  }
+};
+
+// Small graphs (1-D and 2-D to 4-D rows): G lanes per task.  sgd_epoch_kernel2 leaves such a
+// graph bound by one lane's chain - schedule, generator, row loads and the sequential row updates
+// of 10 or so firings one after another, its warp's other lanes diverged - with most of the chip
+// idle (500 points: 27 us per epoch, 32 warps).  Here the lanes of a group evaluate the schedule
+// of 16 entries together, each fetches SLOTS / G of a firing's row slots, one firing ahead of the
+// arithmetic, and all of them apply the updates of the head row, redundantly, with the rows
+// exchanged by shuffles; only the chain of row updates is left.  The warp's 32 / G tasks are
+// neighbours of the layout's order, so they fire about equally often.
+// The draws are those of sgd_epoch_kernel2 (same entry index, epoch and pair).  Rows are read
+// through L2: a launch overlaps the previous epoch's end up to grid_wait, and the schedule of a
+// task's first window, which does not depend on the embedding, is evaluated before it.
+template <int DIM, int G>
+__global__ void __launch_bounds__(256) sgd_epoch_group(
+    const uint64_t* __restrict__ slice_base, const uint32_t* __restrict__ slice_width,
+    const uint32_t* __restrict__ split_mask, const uint32_t* __restrict__ rowid,
+    const uint2* __restrict__ entry, uint64_t n_slices, float* __restrict__ live, float* snap,
+    SgdParams p, uint32_t epoch, float alpha) {
+  constexpr int R = SLOTS / G;  // row slots per lane: slot s belongs to lane s / R
+  __shared__ uint2 s_fire[256 / G][group_window(G) + 1];
+  umma::grid_release();
+  const uint64_t task = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) / G;
+  const uint64_t slice = task >> 5;  // the same for a whole warp
+  if (slice >= n_slices) return;
+  const GroupTask<G> t(slice_base, slice_width, split_mask, rowid, p, slice, task);
+  uint2* fire = s_fire[t.lt];
+  uint32_t m = t.window(entry, 0, epoch, p.neg_rate, fire);
+  umma::grid_wait();
+  float cur[DIM], start[DIM];
+  float* hrow = live + (uint64_t)(t.active ? t.r : 0) * DIM;
+  load_row_l2<DIM>(cur, hrow);
+#pragma unroll
+  for (int d = 0; d < DIM; ++d) start[d] = cur[d];
+
+  float x[R][DIM];       // this lane's slots of the firing at hand
+  uint32_t kk[R];
+  bool ok[R];
+  uint32_t nneg = 0;
+  uint64_t idx = 0;
+  // slots of firing f (of `count`) of the window at ew; `left` holds the window's fires from f on
+  auto fetch = [&](uint32_t f, uint32_t count, uint32_t ew, uint32_t& left, float (&nx)[R][DIM], uint32_t (&nk)[R],
+                   bool (&nok)[R], uint32_t& nn, uint64_t& ni) {
+    const bool has = f < count;
+    const uint2 fe = has ? fire[f] : make_uint2(0u, 0u);
+    nn = fe.y;
+    ni = t.entry_index(ew + (left ? __ffs(left) - 1 : 0));
+    left &= left - 1;
+    const NegRng rng(p.seed, ni, epoch);
+    uint64_t rnd = 0;
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      const uint32_t s = t.gl * R + i;
+      if (i == 0 || (i & 1) == 0) rnd = rng.pair(s >> 1);
+      const uint32_t rv = (s & 1) ? (uint32_t)(rnd >> 32) : (uint32_t)rnd;
+      nk[i] = s == TAIL_SLOT ? fe.x : t.seg_lo + __umulhi(rv, t.seg_n);
+      const bool want = has && (s == TAIL_SLOT || s < nn);
+      nok[i] = want && (s == TAIL_SLOT || nk[i] != t.r);
+      if (want) load_row_l2<DIM>(nx[i], snap + (uint64_t)nk[i] * DIM);
+      else
+#pragma unroll
+        for (int d = 0; d < DIM; ++d) nx[i][d] = 0.0f;
+    }
+  };
+  for (uint32_t ew = 0;;) {
+    __syncwarp();
+    const uint32_t count = (uint32_t)__popc(m);
+    const uint32_t rounds = __reduce_max_sync(0xFFFFFFFFu, count);
+    uint32_t left = m;
+    if (rounds) fetch(0, count, ew, left, x, kk, ok, nneg, idx);
+    for (uint32_t f = 0; f < rounds; ++f) {
+      float nx[R][DIM];
+      uint32_t nk[R], nn = 0;
+      bool nok[R];
+      uint64_t ni = 0;
+      if (f + 1 < rounds) fetch(f + 1, count, ew, left, nx, nk, nok, nn, ni);
+      const bool has = f < count;
+      // attractive step (optimize_layout_euclidean.rs:284-306)
+      {
+        float o[DIM], g[DIM];
+#pragma unroll
+        for (int d = 0; d < DIM; ++d) o[d] = __shfl_sync(0xFFFFFFFFu, x[R - 1][d], G - 1, G);
+        attract<DIM>(cur, o, g, p, alpha);
+        if (has) {
+#pragma unroll
+          for (int d = 0; d < DIM; ++d) cur[d] += g[d];
+          if (t.gl == G - 1) sub_row<DIM>(snap + (uint64_t)kk[R - 1] * DIM, g);
+        }
+      }
+      // negative samples (:313-341)
+      unsigned okb[R];
+#pragma unroll
+      for (int i = 0; i < R; ++i) okb[i] = __ballot_sync(0xFFFFFFFFu, ok[i]) >> t.gshift;
+      const uint32_t nmax = __reduce_max_sync(0xFFFFFFFFu, nneg);
+#pragma unroll
+      for (int q = 0; q < NEG_SLOTS; ++q) {
+        if ((uint32_t)q >= nmax) break;
+        float o[DIM];
+#pragma unroll
+        for (int d = 0; d < DIM; ++d) o[d] = __shfl_sync(0xFFFFFFFFu, x[q % R][d], q / R, G);
+        repel<DIM>(cur, o, (okb[q % R] >> (q / R)) & 1u, p, alpha);
+      }
+      for (uint32_t q = NEG_SLOTS; q < nmax; ++q) {  // more negatives than slots: one at a time
+        float o[DIM];
+        const uint32_t k = negative_row(NegRng(p.seed, idx, epoch), q, t.seg_lo, t.seg_n);
+        const bool apply = q < nneg && k != t.r;
+        if (apply) load_row_l2<DIM>(o, snap + (uint64_t)k * DIM);
+        else
+#pragma unroll
+          for (int d = 0; d < DIM; ++d) o[d] = 0.0f;
+        repel<DIM>(cur, o, apply, p, alpha);
+      }
+#pragma unroll
+      for (int i = 0; i < R; ++i) {
+#pragma unroll
+        for (int d = 0; d < DIM; ++d) x[i][d] = nx[i][d];
+        kk[i] = nk[i];
+        ok[i] = nok[i];
+      }
+      nneg = nn;
+      idx = ni;
+    }
+    ew += group_window(G);
+    if (ew >= t.width) break;
+    __syncwarp();
+    m = t.window(entry, ew, epoch, p.neg_rate, fire);
+  }
+  if (t.active && t.gl == 0) {
+    if (t.split) {
+#pragma unroll
+      for (int d = 0; d < DIM; ++d) atomicAdd(hrow + d, cur[d] - start[d]);
+    } else {
+      store_row<DIM>(hrow, cur);
+    }
+  }
+}
+
+// Rows of more than 4 columns (n_components 5 to 128): a group of G lanes per task, lane j holding
+// columns j, j + G, ... (C of them) of the head row in registers, so a row is one coalesced read and
+// a squared distance one shuffle reduction.  The schedule, the generator (lane q draws negative q)
+// and the fetch of a firing's rows one firing ahead are those of sgd_epoch_group.  A thread per task
+// with its head row in global memory (sgd_epoch_anydim) pays a dependent global round trip for
+// every column of every update.
+template <int G, int C, bool GEN>
+__global__ void __launch_bounds__(256) sgd_epoch_columns(
+    const uint64_t* __restrict__ slice_base, const uint32_t* __restrict__ slice_width,
+    const uint32_t* __restrict__ split_mask, const uint32_t* __restrict__ rowid,
+    const uint2* __restrict__ entry, uint64_t n_slices, float* __restrict__ live, float* snap,
+    SgdParams p, uint32_t epoch, float alpha) {
+  constexpr int NS = 8;  // rows fetched ahead: the first 7 negatives and the tail
+  __shared__ uint2 s_fire[256 / G][group_window(G) + 1];
+  umma::grid_release();
+  const uint64_t task = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) / G;
+  const uint64_t slice = task >> 5;
+  if (slice >= n_slices) return;
+  const GroupTask<G> t(slice_base, slice_width, split_mask, rowid, p, slice, task);
+  uint2* fire = s_fire[t.lt];
+  uint32_t m = t.window(entry, 0, epoch, p.neg_rate, fire);
+  umma::grid_wait();
+  const uint32_t dim = p.dim;
+  float cur[C], start[C];
+  float* hrow = live + (uint64_t)(t.active ? t.r : 0) * dim;
+  // this lane's columns of a row (0 where there is none)
+  auto load = [&](float (&v)[C], const float* row, bool want) {
+#pragma unroll
+    for (int i = 0; i < C; ++i) {
+      const uint32_t c = t.gl + i * G;
+      v[i] = want && c < dim ? __ldcg(row + c) : 0.0f;
+    }
+  };
+  load(cur, hrow, t.active);
+#pragma unroll
+  for (int i = 0; i < C; ++i) start[i] = cur[i];
+
+  auto square = [&](const float (&df)[C]) {
+    float ds = t.gl == 0 ? 1.17549435e-38f : 0.0f;  // as in square_ftz
+#pragma unroll
+    for (int i = 0; i < C; ++i) ds = fmaf(df[i], df[i], ds);
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1) ds += __shfl_xor_sync(0xFFFFFFFFu, ds, o);
+    return ds;
+  };
+  auto repel = [&](const float (&o)[C], bool apply) {
+    float df[C];
+#pragma unroll
+    for (int i = 0; i < C; ++i) df[i] = cur[i] - o[i];
+    const float ds = square(df);
+    if constexpr (GEN) {
+      float den;
+      const float gr = metric_coeff(ds, p.a, p.two_b, p.pos_rep, 0.0f, &den);
+      if (apply) {
+#pragma unroll
+        for (int i = 0; i < C; ++i) cur[i] += clip4(gr * __fdividef(df[i], den)) * alpha;
+      }
+    } else {
+      const float inv = repel_inv(ds, p);
+      if (apply && ds > 0.0f) {
+#pragma unroll
+        for (int i = 0; i < C; ++i) cur[i] = fmaf(clip4((p.pos_rep * df[i]) * inv), alpha, cur[i]);
+      }
+    }
+  };
+  float x[NS][C];
+  uint32_t kk = 0, nneg = 0;
+  uint64_t idx = 0;
+  auto fetch = [&](uint32_t f, uint32_t count, uint32_t ew, uint32_t& left, float (&nx)[NS][C], uint32_t& nk,
+                   uint32_t& nn, uint64_t& ni) {
+    const bool has = f < count;
+    const uint2 fe = has ? fire[f] : make_uint2(0u, 0u);
+    nn = fe.y;
+    ni = t.entry_index(ew + (left ? __ffs(left) - 1 : 0));
+    left &= left - 1;
+    nk = t.gl == NS - 1 ? fe.x : negative_row(NegRng(p.seed, ni, epoch), t.gl, t.seg_lo, t.seg_n);
+#pragma unroll
+    for (int s = 0; s < NS; ++s) {
+      const uint32_t k = __shfl_sync(0xFFFFFFFFu, nk, s, G);
+      load(nx[s], snap + (uint64_t)k * dim, has && (s == NS - 1 || (uint32_t)s < nn));
+    }
+  };
+
+  for (uint32_t ew = 0;;) {
+    __syncwarp();
+    const uint32_t count = (uint32_t)__popc(m);
+    const uint32_t rounds = __reduce_max_sync(0xFFFFFFFFu, count);
+    uint32_t left = m;
+    if (rounds) fetch(0, count, ew, left, x, kk, nneg, idx);
+    for (uint32_t f = 0; f < rounds; ++f) {
+      float nx[NS][C];
+      uint32_t nk = 0, nn = 0;
+      uint64_t ni = 0;
+      if (f + 1 < rounds) fetch(f + 1, count, ew, left, nx, nk, nn, ni);
+      const bool has = f < count;
+      {
+        float df[C];
+#pragma unroll
+        for (int i = 0; i < C; ++i) df[i] = cur[i] - x[NS - 1][i];
+        const float ds = square(df);
+        float gc, inv;
+        if constexpr (GEN) {
+          float den;
+          gc = metric_coeff(ds, p.a, p.two_b, p.two_b, -1.0f, &den);
+          inv = __fdividef(1.0f, den);
+        } else {
+          attract_terms(ds, p, gc, inv);
+        }
+        const uint32_t k = __shfl_sync(0xFFFFFFFFu, kk, NS - 1, G);
+        if (has) {
+#pragma unroll
+          for (int i = 0; i < C; ++i) {
+            const float g = clip4((gc * df[i]) * inv) * alpha;
+            cur[i] += g;
+            const uint32_t c = t.gl + i * G;
+            if (c < dim) atomicAdd(snap + (uint64_t)k * dim + c, -g);
+          }
+        }
+      }
+      const uint32_t nmax = __reduce_max_sync(0xFFFFFFFFu, nneg);
+      const unsigned okb = __ballot_sync(0xFFFFFFFFu, t.gl < NS - 1 && t.gl < nneg && kk != t.r) >> t.gshift;
+#pragma unroll
+      for (int q = 0; q < NS - 1; ++q) {
+        if ((uint32_t)q >= nmax) break;
+        repel(x[q], (okb >> q) & 1u);
+      }
+      for (uint32_t q = NS - 1; q < nmax; ++q) {
+        float o[C];
+        const uint32_t k = negative_row(NegRng(p.seed, idx, epoch), q, t.seg_lo, t.seg_n);
+        const bool apply = q < nneg && k != t.r;
+        load(o, snap + (uint64_t)k * dim, apply);
+        repel(o, apply);
+      }
+      if (t.split && has) {  // a partial row: merge this firing's moves with the other parts' so far
+#pragma unroll
+        for (int i = 0; i < C; ++i) {
+          const uint32_t c = t.gl + i * G;
+          if (c >= dim) continue;
+          const float moved = cur[i] - start[i];
+          cur[i] = start[i] = atomicAdd(hrow + c, moved) + moved;
+        }
+      }
+#pragma unroll
+      for (int s = 0; s < NS; ++s)
+#pragma unroll
+        for (int i = 0; i < C; ++i) x[s][i] = nx[s][i];
+      kk = nk;
+      nneg = nn;
+      idx = ni;
+    }
+    ew += group_window(G);
+    if (ew >= t.width) break;
+    __syncwarp();
+    m = t.window(entry, ew, epoch, p.neg_rate, fire);
+  }
+  if (t.active) {
+#pragma unroll
+    for (int i = 0; i < C; ++i) {
+      const uint32_t c = t.gl + i * G;
+      if (c < dim && !t.split) hrow[c] = cur[i];
     }
   }
 }
@@ -611,9 +1092,8 @@ __global__ void slice_meta_kernel(const uint32_t* __restrict__ perm, const uint3
   // slice width = longest task of the slice (instance-major order: the max over lanes)
   uint32_t len = q < T ? chunk - ((skey[q] >> rate_bits) & len_mask) : 0u;
   for (int o = 16; o > 0; o >>= 1) len = max(len, __shfl_xor_sync(0xFFFFFFFFu, len, o));
-  // whole register windows per lane (UB_SGD2_W entries, a multiple of one 4-entry sector): the
-  // lane-major epoch loads a full window without a bounds check
-  if (lane_major) len = (len + (UB_SGD2_W - 1u)) / UB_SGD2_W * UB_SGD2_W;
+  // whole 32-byte sectors per task
+  if (lane_major) len = (len + 3u) / 4u * 4u;
   if ((q & 31) == 0) {
     width[q >> 5] = len;
     split_mask[q >> 5] = bits;
@@ -916,45 +1396,49 @@ uint32_t pick_chunk_generic(uint64_t n_edges) {
   return std::max<uint32_t>(64, pick_chunk(n_edges));
 }
 
-// Whether the epoch kernel takes the 8-negatives budget (the Euclidean rule in 2-D and 1-D):
-// where the layout's warps (one per slice) fill at most two waves of the wide budget's
-// resident warps (SMs x 5 blocks x 8 warps), and for renamed DRAM-bound layouts, where more
-// row loads in flight per lane hide DRAM latency (20M-point swiss roll, 30 epochs: 337.7 ->
-// 308.4 ms).  UMAP_B200_SGD_SHORT=0 / 1 forces it.
-bool pick_short_epoch(uint64_t n_slices, bool renamed) {
-  if (const char* e = getenv("UMAP_B200_SGD_SHORT")) {
-    if (e[0] == '0') return false;
-    if (e[0] == '1') return true;
-  }
-  if (renamed) return true;  // the layout takes the DRAM budget (pick_dram_epoch) unless forced
+// Graphs of at most two waves of a lane per task at 40 warps per SM: their tasks are ordered by firing
+// rate too (pick_task_order).
+bool small_graph(uint64_t n_slices) {
   int dev = 0, sms = 0;
   UB_CUDA(cudaGetDevice(&dev));
   UB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  return n_slices <= 2ull * (uint64_t)std::max(sms, 1) * MINB_WIDE * 8;
+  return n_slices <= 2ull * (uint64_t)std::max(sms, 1) * 40;
 }
 
-// Renamed (DRAM-bound) layouts take the 12-negatives budget unless UMAP_B200_SGD_SHORT forces one
-// of the other two.
-bool pick_dram_epoch(bool renamed) {
-  return renamed && getenv("UMAP_B200_SGD_SHORT") == nullptr;
-}
-
-// Entry order of the layout.  Lane major (a lane's window is one 32-byte sector) wins while
-// the rows the negatives and tails reach stay in L2: a plain fit whose 2-D embedding (live +
-// snapshot, 16 B per vertex) is at most 64 MB, and batched instances, whose instance-major
-// task order keeps the instances in flight in L2.  Beyond that every access goes to DRAM,
-// where the interleaved order's whole 256-byte rows per warp use DRAM bursts better than
-// 32-byte windows.  UMAP_B200_SGD_LANE_MAJOR=0 / 1 forces either.
-bool pick_lane_major(uint64_t n, bool segmented) {
-  if (const char* e = getenv("UMAP_B200_SGD_LANE_MAJOR")) {
-    if (e[0] == '0') return false;
-    if (e[0] == '1') return true;
+// The epoch kernel of a layout.
+//  * Columns / AnyDim: rows of 5 to 128 and of more columns.
+//  * Dram: renamed 1-D and 2-D layouts whose snapshot (4 * dim bytes per vertex) is above 80 MB, so
+//    that with the edge stream it does not stay in the 126 MB L2.  The random rows then cost DRAM
+//    bursts, and the interleaved order's whole 256-byte rows per warp use them better than a task's
+//    contiguous entries (2-D rolls, 30 epochs, Dram interleaved against Pool lane major, ms: 5M points
+//    34.7 / 28.2, 8M 55.1 / 44.6, 12M 94.6 / 98.7, 16M 149.6 / 156.9, 20M 207.2 / 221.6).
+//  * Group8 / Group4: G lanes per task while T tasks of G lanes are at most about 1,450 threads per
+//    SM (2-D mixtures, k = 15, us per epoch, Group8 / Group4 / Pool: 500 points 12.2 / 13.9 / 19.9,
+//    10k 18.5 / 22.7 / 24.3, 14k 20.2 / 22.0 / 24.6, 22k 26.7 / 22.7 / 26.1, 30k 34.0 / 27.4 / 27.6,
+//    70k 70 / 47 / 34).
+//  * Pool: everything else, and the generic-metric rule at every size.
+// UMAP_B200_SGD_KERNEL=pool / group4 / group8 / dram forces one that can run the layout.
+EpochKernel pick_epoch_kernel(uint64_t n, uint32_t dim, uint64_t n_tasks, bool renamed, bool segmented, bool generic) {
+  if (dim > 128) return EpochKernel::AnyDim;
+  if (dim > 4) return EpochKernel::Columns;
+  const bool can_dram = dim <= 2 && !generic && !segmented;
+  if (const char* e = getenv("UMAP_B200_SGD_KERNEL")) {
+    if (!strcmp(e, "dram") && can_dram) return EpochKernel::Dram;
+    if (!strcmp(e, "pool")) return EpochKernel::Pool;
+    if (!strcmp(e, "group4") && !generic) return EpochKernel::Group4;
+    if (!strcmp(e, "group8") && !generic) return EpochKernel::Group8;
   }
-  return segmented || n <= 4000000ull;
+  if (can_dram && renamed && n * dim * 4 > 80000000ull) return EpochKernel::Dram;
+  if (generic) return EpochKernel::Pool;
+  int dev = 0, sms = 0;
+  UB_CUDA(cudaGetDevice(&dev));
+  UB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  const uint64_t room = 1450ull * (uint64_t)std::max(sms, 1);
+  return n_tasks * 8 <= room ? EpochKernel::Group8 : n_tasks * 4 <= room ? EpochKernel::Group4 : EpochKernel::Pool;
 }
 
-// Whether a plain fit's layout renames its vertices into a locality order (order.cu): where
-// every random access is a DRAM access, i.e. the sizes that take interleaved entries.
+// Whether a plain fit's layout renames its vertices into a locality order (order.cu): from the
+// sizes at which random rows of the caller's order mostly miss L2.
 // UMAP_B200_RELABEL=0 / 1 forces either.  The generic-metric rule never renames (its caller
 // passes rename = false): it is sensitive to which rows update at the same time (its split
 // rows showed that), and its parity with the reference was established in the caller's order;
@@ -998,13 +1482,12 @@ TaskOrder pick_task_order(bool renamed, bool short_graph, bool segmented) {
   return short_graph ? TaskOrder::LengthRate : TaskOrder::Length;
 }
 
-void build_sgd_layout(const uint64_t* kept_ptr, const uint32_t* ktail, const double* keps, uint64_t n,
-                      uint32_t chunk, SgdLayout& L, cudaStream_t s, const Segments* seg, bool rename) {
+void build_sgd_layout(const uint64_t* kept_ptr, const uint32_t* ktail, const double* keps, uint64_t n, uint32_t dim,
+                      uint32_t chunk, bool generic, SgdLayout& L, cudaStream_t s, const Segments* seg) {
   L.n_vertices = n;
-  L.lane_major = pick_lane_major(n, seg != nullptr);
   DevBuf<uint32_t> rank;
   L.order.reset();
-  if (n && rename && pick_relabel(n, seg != nullptr)) {
+  if (n && !generic && pick_relabel(n, seg != nullptr)) {
     L.order.alloc(n, s);
     rank.alloc(n, s);
     locality_order(kept_ptr, ktail, n, L.order.p, rank.p, s);
@@ -1013,7 +1496,7 @@ void build_sgd_layout(const uint64_t* kept_ptr, const uint32_t* ktail, const dou
   UB_CUDA(cudaMemcpyAsync(&n_edges, kept_ptr + n, 8, cudaMemcpyDeviceToHost, s));
   UB_CUDA(cudaStreamSynchronize(s));
   L.n_edges = n_edges;
-  L.chunk = chunk ? chunk : pick_chunk(n_edges);
+  L.chunk = chunk ? chunk : generic ? pick_chunk_generic(n_edges) : pick_chunk(n_edges);
   DevBuf<uint32_t> deg(n, s), ntask(n, s);
   if (n) {
     ptr_degree_kernel<<<grid_for(n, 256), 256, 0, s>>>(kept_ptr, n, L.chunk, L.order.p, deg.p, ntask.p);
@@ -1037,7 +1520,9 @@ void build_sgd_layout(const uint64_t* kept_ptr, const uint32_t* ktail, const dou
   if ((uint64_t)n_seg << len_bits >= (1ull << 32)) throw Error(UNSUPPORTED, "too many instances for the task sort key");
   const int seg_bits = n_seg ? bits_for(n_seg) : 0;
   const bool renamed = L.order.p != nullptr;
-  TaskOrder torder = pick_task_order(renamed, pick_short_epoch((T + 31) / 32, renamed), seg != nullptr);
+  L.kernel = pick_epoch_kernel(n, dim, T, renamed, seg != nullptr, generic);
+  L.lane_major = L.kernel != EpochKernel::Dram;
+  TaskOrder torder = pick_task_order(renamed, small_graph((T + 31) / 32), seg != nullptr);
   if (torder == TaskOrder::LengthRate && len_bits + seg_bits + RATE_BITS > 32) torder = TaskOrder::Length;
   L.task_order = torder;
   const int rate_bits = torder == TaskOrder::LengthRate ? RATE_BITS : 0;
@@ -1097,8 +1582,6 @@ void build_sgd_layout(const uint64_t* kept_ptr, const uint32_t* ktail, const dou
   UB_CUDA(cudaStreamSynchronize(s));
   L.split_tasks = 0;
   for (uint32_t v : h) L.split_tasks += __builtin_popcount(v);
-  L.short_epoch = pick_short_epoch(L.n_slices, L.order.p != nullptr);
-  L.dram_epoch = pick_dram_epoch(L.order.p != nullptr);
 }
 
 void export_edges(const uint64_t* indptr, const uint32_t* indices, const float* data, uint64_t n,
@@ -1131,46 +1614,82 @@ void normalize_init(float* emb, uint64_t n, uint32_t dim, cudaStream_t s, const 
   UB_LAUNCH_CHECK();
 }
 
+uint32_t epoch_block_threads(const SgdLayout& L) { return L.kernel == EpochKernel::Pool ? POOL_BT : 256; }
+
+// Launches an epoch kernel; `overlap` makes it a programmatic dependent of the launch before it on
+// the stream (only kernels that wait for that launch with grid_wait take it).
+template <class... P, class... A>
+void launch_epoch(void (*k)(P...), unsigned grid, unsigned bt, bool overlap, cudaStream_t s, A&&... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(bt);
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = overlap ? 1 : 0;
+  UB_CUDA(cudaLaunchKernelEx(&cfg, k, std::forward<A>(args)...));
+  count_launch();
+}
+
+// The launch may overlap the end of the epoch before it (`overlap`): every kernel but Dram and AnyDim
+// evaluates its schedule before grid_wait.  A small launch is released to the next one when its
+// blocks start - the next epoch's blocks find free slots - and so is a large one (2M points: 474
+// against 484 us per epoch); the pooled kernel in between releases at its blocks' end, since the next
+// epoch's early blocks would fill the SMs unevenly (70k points: 34 against 41 us).
 void sgd_epoch(const SgdLayout& L, float* live, float* snap, const SgdParams& p, uint32_t epoch, float alpha,
-               cudaStream_t s) {
+               bool overlap, cudaStream_t s) {
   if (L.n_slices == 0) return;
-  const unsigned bt = L.block_threads ? L.block_threads : 256;
-  const unsigned grid = grid_for(L.n_slices * 32, bt);
+  constexpr unsigned BT = 256;
+  const uint64_t tasks = L.n_slices * 32;
+  auto blocks = [](uint64_t threads, unsigned bt) {
+    const uint64_t g = (threads + bt - 1) / bt;
+    if (g > 0x7FFFFFFFull) throw Error(UNSUPPORTED, "too many SGD tasks for one launch");
+    return (unsigned)g;
+  };
 #define UB_SGD_ARGS L.slice_base.p, L.slice_width.p, L.split_mask.p, L.rowid.p, L.entry.p, L.n_slices, live, snap, \
                     p, epoch, alpha
-#define UB_SGD_WIDE(D, GEN)                                                                   \
-  if (L.lane_major) sgd_epoch_kernel2<D, GEN, NB_WIDE, MINB_WIDE, true><<<grid, bt, 0, s>>>(UB_SGD_ARGS); \
-  else sgd_epoch_kernel2<D, GEN, NB_WIDE, MINB_WIDE, false><<<grid, bt, 0, s>>>(UB_SGD_ARGS)
-// short graphs are small, so lane major by default (pick_lane_major); both orders are built
-#define UB_SGD_SHORT(D, GEN)                                                                    \
-  if (L.lane_major) sgd_epoch_kernel2<D, GEN, NB_SHORT, MINB_SHORT, true><<<grid, bt, 0, s>>>(UB_SGD_ARGS); \
-  else sgd_epoch_kernel2<D, GEN, NB_SHORT, MINB_SHORT, false><<<grid, bt, 0, s>>>(UB_SGD_ARGS)
-#define UB_SGD_DISPATCH(GEN, SHORT)                                                   \
-  switch (p.dim) {                                                                    \
-    case 1: if (SHORT) UB_SGD_SHORT(1, GEN); else UB_SGD_WIDE(1, GEN); break;         \
-    case 2: if (SHORT) UB_SGD_SHORT(2, GEN); else UB_SGD_WIDE(2, GEN); break;         \
-    case 3: UB_SGD_WIDE(3, GEN); break;                                               \
-    case 4: UB_SGD_WIDE(4, GEN); break;                                               \
-    default: sgd_epoch_anydim<GEN><<<grid, bt, 0, s>>>(UB_SGD_ARGS, L.lane_major); break; \
+  auto grouped = [&](auto k, uint32_t lanes) { launch_epoch(k, blocks(tasks * lanes, BT), BT, overlap, s, UB_SGD_ARGS); };
+  auto pooled = [&](auto k) {
+    const unsigned g = blocks(tasks, POOL_BT);
+    launch_epoch(k, g, POOL_BT, overlap, s, UB_SGD_ARGS, g > 8000u);
+  };
+  const bool gen = p.generic_metric;
+  switch (L.kernel) {
+    case EpochKernel::Group8:
+      if (p.dim == 1) grouped(sgd_epoch_group<1, 8>, 8);
+      else if (p.dim == 2) grouped(sgd_epoch_group<2, 8>, 8);
+      else if (p.dim == 3) grouped(sgd_epoch_group<3, 8>, 8);
+      else grouped(sgd_epoch_group<4, 8>, 8);
+      break;
+    case EpochKernel::Group4:
+      if (p.dim == 1) grouped(sgd_epoch_group<1, 4>, 4);
+      else if (p.dim == 2) grouped(sgd_epoch_group<2, 4>, 4);
+      else if (p.dim == 3) grouped(sgd_epoch_group<3, 4>, 4);
+      else grouped(sgd_epoch_group<4, 4>, 4);
+      break;
+    case EpochKernel::Pool:
+      if (p.dim == 1) gen ? pooled(sgd_epoch_pool<1, true>) : pooled(sgd_epoch_pool<1, false>);
+      else if (p.dim == 2) gen ? pooled(sgd_epoch_pool<2, true>) : pooled(sgd_epoch_pool<2, false>);
+      else if (p.dim == 3) gen ? pooled(sgd_epoch_pool<3, true>) : pooled(sgd_epoch_pool<3, false>);
+      else gen ? pooled(sgd_epoch_pool<4, true>) : pooled(sgd_epoch_pool<4, false>);
+      break;
+    case EpochKernel::Columns:
+      if (p.dim <= 8) gen ? grouped(sgd_epoch_columns<8, 1, true>, 8) : grouped(sgd_epoch_columns<8, 1, false>, 8);
+      else if (p.dim <= 16) gen ? grouped(sgd_epoch_columns<16, 1, true>, 16) : grouped(sgd_epoch_columns<16, 1, false>, 16);
+      else if (p.dim <= 32) gen ? grouped(sgd_epoch_columns<32, 1, true>, 32) : grouped(sgd_epoch_columns<32, 1, false>, 32);
+      else if (p.dim <= 64) gen ? grouped(sgd_epoch_columns<32, 2, true>, 32) : grouped(sgd_epoch_columns<32, 2, false>, 32);
+      else gen ? grouped(sgd_epoch_columns<32, 4, true>, 32) : grouped(sgd_epoch_columns<32, 4, false>, 32);
+      break;
+    case EpochKernel::Dram:
+      launch_epoch(p.dim == 1 ? sgd_epoch_dram<1> : sgd_epoch_dram<2>, blocks(tasks, BT), BT, false, s, UB_SGD_ARGS);
+      break;
+    case EpochKernel::AnyDim:
+      launch_epoch(gen ? sgd_epoch_anydim<true> : sgd_epoch_anydim<false>, blocks(tasks, BT), BT, false, s, UB_SGD_ARGS);
+      break;
   }
-  // The generic-metric rule keeps the large-graph budget at every size (its statistical
-  // parity with the reference's sequential loop was established with it).
-  if (p.generic_metric) {
-    UB_SGD_DISPATCH(true, false)
-  } else if (L.dram_epoch && (p.dim == 1 || p.dim == 2)) {
-#define UB_SGD_DRAM(D)                                                                                       \
-  if (L.lane_major) sgd_epoch_kernel2<D, false, NB_DRAM, MINB_DRAM, true><<<grid, bt, 0, s>>>(UB_SGD_ARGS); \
-  else sgd_epoch_kernel2<D, false, NB_DRAM, MINB_DRAM, false><<<grid, bt, 0, s>>>(UB_SGD_ARGS)
-    if (p.dim == 1) { UB_SGD_DRAM(1); } else { UB_SGD_DRAM(2); }
-#undef UB_SGD_DRAM
-  } else {
-    UB_SGD_DISPATCH(false, L.short_epoch)
-  }
-#undef UB_SGD_DISPATCH
-#undef UB_SGD_SHORT
-#undef UB_SGD_WIDE
 #undef UB_SGD_ARGS
-  UB_LAUNCH_CHECK();
 }
 
 void schedule_totals(const SgdLayout& L, uint32_t neg_rate, uint32_t start, uint32_t end,

@@ -181,12 +181,13 @@ constexpr uint64_t MAX_EPOCHS = 1ull << 21;
 // Order in which build_sgd_layout deals tasks to warps (sgd.cu, pick_task_order).
 enum class TaskOrder { Length, LengthRate, RowBlock, Row };
 
+// Which kernel runs the layout's epochs (sgd.cu, pick_epoch_kernel).
+enum class EpochKernel { Pool, Group8, Group4, Columns, AnyDim, Dram };
+
 struct SgdLayout {
   uint64_t n_vertices = 0, n_edges = 0, n_entries = 0, n_slices = 0, n_tasks = 0;
   uint32_t max_degree = 0, chunk = 0;
-  uint32_t block_threads = 256;  // threads per block of the epoch kernel (multiple of 32)
-  bool short_epoch = false;      // epoch kernel budget for graphs of at most ~2 waves of warps
-  bool dram_epoch = false;       // 12-negatives budget of renamed DRAM-bound layouts
+  EpochKernel kernel = EpochKernel::Pool;
   bool lane_major = true;        // entry order: lane major (true) or interleaved by lane
   TaskOrder task_order = TaskOrder::Length;
   uint64_t split_tasks = 0;
@@ -252,17 +253,19 @@ uint32_t pick_chunk(uint64_t n_edges);
 uint32_t pick_chunk_generic(uint64_t n_edges);
 // `rename`: a plain fit's layout may rename its vertices into a locality order (DRAM-bound
 // sizes); the generic-metric rule passes false.
-void build_sgd_layout(const uint64_t* kept_ptr, const uint32_t* tail, const double* eps,
-                      uint64_t n, uint32_t chunk, SgdLayout& L, cudaStream_t s,
-                      const Segments* seg = nullptr, bool rename = true);
+void build_sgd_layout(const uint64_t* kept_ptr, const uint32_t* tail, const double* eps, uint64_t n, uint32_t dim,
+                      uint32_t chunk, bool generic, SgdLayout& L, cudaStream_t s, const Segments* seg = nullptr);
+// Threads per block of the layout's epoch kernel.
+uint32_t epoch_block_threads(const SgdLayout& L);
 void kept_degree(const uint64_t* indptr, const float* data, uint64_t n, float thr,
                  uint32_t* deg, cudaStream_t s, const SegmentPrune* sp = nullptr);
 // K6 normalise init into [0, 10] per dimension (optimizer.rs:181-230), in place.
 void normalize_init(float* emb, uint64_t n, uint32_t dim, cudaStream_t s,
                     const Segments* seg = nullptr);
-// K7 one Hogwild epoch.
+// K7 one Hogwild epoch.  `overlap`: the launch before it on the stream is an epoch of the same
+// layout and buffers, whose end it may overlap (where the kernel can).
 void sgd_epoch(const SgdLayout& L, float* live, float* snap, const SgdParams& p,
-               uint32_t epoch, float alpha, cudaStream_t s);
+               uint32_t epoch, float alpha, bool overlap, cudaStream_t s);
 // Exact totals of fired edges / negatives over epochs [start, end).
 // Warm-start row helpers (warm.cu): rows (or rows[i]) of x [*, d] zero-padded to dp columns;
 // keep[r] = 1 for rows of y [n, dim] without NaN/inf; rows with keep set moved to pos[r].
