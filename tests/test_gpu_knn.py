@@ -104,3 +104,21 @@ def test_knn_feeds_the_fit(ub, oracle):
     G = m.graph()
     ip, ix, _ = mo.graph()
     assert np.array_equal(G.indptr, ip) and np.array_equal(G.indices, ix)
+
+
+@pytest.mark.parametrize("n,d,k,kind", [
+    (2048, 16, 33, "gauss"), (2049, 40, 128, "clusters"), (2300, 3, 64, "ties"), (3000, 100, 65, "pixels"),
+    (5000, 24, 100, "offset"), (16384, 8, 40, "clusters"), (17001, 20, 128, "gauss"), (2500, 2, 100, "lines"),
+])
+def test_knn_long_lists_candidate_pass(ub, oracle, n, d, k, kind):
+    """k above 32 from 2,048 points: candidates of 4 or 8 database splits, ranks dealt over their lists
+    (whole and partial groups of tiles), rows whose lists overflow recomputed ("lines": 20 points
+    repeated 125 times, far more equal distances than a list holds)."""
+    if kind == "lines":
+        X = np.repeat(_data(20, d, seed=1), n // 20, axis=0)
+    else:
+        X = _data(n, d, seed=n + k, kind=kind)
+    gi, gd, rec = ub.knn_bruteforce(X, k, return_stats=True)
+    oi, od = oracle.knn_bruteforce(X, k)
+    assert np.array_equal(gi, oi) and np.array_equal(gd, od), rec
+    assert kind in ("lines", "ties") or rec < n // 20, rec

@@ -219,8 +219,8 @@ def batch_fit(config: UmapConfig, offsets, knn_indices, knn_dists, init):
     return out
 
 
-KNN_MAX_K = 128       # largest k; above 32 every row takes the exact CUDA-core path
-KNN_MAX_K_TENSOR = 32  # largest k through the tensor-core candidate pass
+KNN_MAX_K = 128       # largest k
+KNN_MAX_K_TENSOR = 32  # largest k through the tensor-core candidate pass at every size (longer from 2,048 rows)
 
 
 def knn_bruteforce(data, k: int, return_stats: bool = False):
