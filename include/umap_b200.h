@@ -261,10 +261,10 @@ int umap_batch_fit_device(const umap_config* cfg, uint64_t n_instances, const ui
 int umap_optimizer_tuning(const umap_optimizer* opt, uint32_t* chunk, uint32_t* block_threads);
 /* Extension: how the SGD layout is laid out (bit flags): UMAP_LAYOUT_LANE_MAJOR (a lane's
  * edges contiguous; else interleaved by lane), the epoch kernel: UMAP_LAYOUT_POOLED (a thread per
- * task, tasks dealt by firings in blocks of 128), UMAP_LAYOUT_GROUP_4 / _GROUP_8 (4 or 8 lanes per
- * task; small graphs), UMAP_LAYOUT_COLUMNS (5 to 128 components, lanes over columns),
+ * task, tasks dealt by firings in blocks of 128), UMAP_LAYOUT_ROWS (a thread per task;
+ * 5 to 7 components),
  * UMAP_LAYOUT_DRAM with _TWELVE_NEGATIVES (a lane per task, 12 row loads in flight; DRAM-bound layouts),
- * none of them: more than 128 components; UMAP_LAYOUT_EIGHT_NEGATIVES (no longer set),
+ * none of them: any number of components; UMAP_LAYOUT_EIGHT_NEGATIVES (no longer set),
  * UMAP_LAYOUT_RENAMED (vertices renamed into a locality
  * order; DRAM-bound plain fits), UMAP_LAYOUT_GENERIC_RULE (the optimizer's MetricType is
  * Generic), and the order in which tasks are dealt to warps: UMAP_LAYOUT_RATE_ORDER (by
@@ -280,10 +280,8 @@ int umap_optimizer_tuning(const umap_optimizer* opt, uint32_t* chunk, uint32_t* 
 #define UMAP_LAYOUT_BLOCK_ORDER 64u
 #define UMAP_LAYOUT_ROW_ORDER 128u
 #define UMAP_LAYOUT_POOLED 256u
-#define UMAP_LAYOUT_GROUP_4 512u
-#define UMAP_LAYOUT_GROUP_8 1024u
-#define UMAP_LAYOUT_COLUMNS 2048u
-#define UMAP_LAYOUT_DRAM 4096u
+#define UMAP_LAYOUT_ROWS 512u
+#define UMAP_LAYOUT_DRAM 1024u
 int umap_optimizer_layout_flags(const umap_optimizer* opt, uint32_t* flags);
 
 /* ---- serde checkpoints (optimizer.rs:27, manifold.rs:14, embedding.rs:438) ---------

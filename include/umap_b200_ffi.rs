@@ -25,10 +25,8 @@ pub const UMAP_LAYOUT_RATE_ORDER: u32 = 32;
 pub const UMAP_LAYOUT_BLOCK_ORDER: u32 = 64;
 pub const UMAP_LAYOUT_ROW_ORDER: u32 = 128;
 pub const UMAP_LAYOUT_POOLED: u32 = 256;
-pub const UMAP_LAYOUT_GROUP_4: u32 = 512;
-pub const UMAP_LAYOUT_GROUP_8: u32 = 1024;
-pub const UMAP_LAYOUT_COLUMNS: u32 = 2048;
-pub const UMAP_LAYOUT_DRAM: u32 = 4096;
+pub const UMAP_LAYOUT_ROWS: u32 = 512;
+pub const UMAP_LAYOUT_DRAM: u32 = 1024;
 pub const UMAP_WARM_START_PHASES: usize = 8;
 
 #[repr(C)]

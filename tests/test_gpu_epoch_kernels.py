@@ -39,9 +39,7 @@ def _steps(ub, cfg, idx, dist, init, epochs, steps):
     return opt.embedding(), opt.layout()
 
 
-KERNELS = [("pool", 1), ("pool", 2), ("pool", 3), ("pool", 4), ("group4", 2), ("group8", 1), ("group8", 2), ("group8", 3),
-           ("group8", 4), ("dram", 1), ("dram", 2), ("", 5), ("", 8), ("", 9), ("", 17), ("", 33), ("", 65), ("", 128),
-           ("", 129)]
+KERNELS = [("pool", 1), ("pool", 2), ("pool", 3), ("pool", 4), ("dram", 1), ("dram", 2), ("", 5), ("", 6), ("", 7), ("", 8), ("", 33)]
 
 
 def _spread(init, dim):
@@ -63,7 +61,7 @@ def test_sequential_rows_match_oracle(ub, oracle, monkeypatch, kernel, dim):
     if kernel:
         monkeypatch.setenv("UMAP_B200_SGD_KERNEL", kernel)
     got, layout = _steps(ub, _config(ub, dim, 12, 0, 0.1), idx, dist, init, 12, (7, 5))
-    assert kernel.rstrip("48") in layout["kernel"]
+    assert kernel in layout["kernel"]
     ocfg = oracle.OracleConfig(n_neighbors=K, negative_sample_rate=0, n_epochs=12, learning_rate=0.1, symmetrize=False,
                                n_components=dim)
     oo = oracle.Optimizer(oracle.learn_manifold(idx, dist, ocfg), init, 12, ocfg, seed=1)
@@ -77,20 +75,18 @@ def test_sequential_rows_match_oracle(ub, oracle, monkeypatch, kernel, dim):
 
 @pytest.mark.parametrize("chunk", ["64", "16"])
 @pytest.mark.parametrize("neg", [5, 20])
-@pytest.mark.parametrize("kernel,dim", [k for k in KERNELS if k[0] in ("group4", "group8", "")])
+@pytest.mark.parametrize("kernel,dim", [k for k in KERNELS if k[0] != "dram" and k[1] > 1 and k != ("pool", 2)])
 def test_negatives_are_the_same_draws(ub, monkeypatch, kernel, dim, neg, chunk):
     """The kernels draw the same negatives (same entry, epoch and pair), so a fit with two live
     columns, the others all zero, moves them as the pooled 2-D kernel does.  At rate 1e-4 a
     racing read differs by one move (4e-4 at most), which changes a later move by under 1e-4 of
     it times the repulsion's slope (below 1,800): within 1e-4."""
-    if dim == 1:
-        pytest.skip("a 2-D embedding needs two columns")
     idx, dist, init = _stars(3)
     monkeypatch.setenv("UMAP_B200_CHUNK", chunk)
     monkeypatch.setenv("UMAP_B200_SGD_KERNEL", "pool")
     want, _ = _steps(ub, _config(ub, 2, 12, neg, 1e-4), idx, dist, init, 12, (1,) * 6)
     monkeypatch.setenv("UMAP_B200_SGD_KERNEL", kernel)
     got, layout = _steps(ub, _config(ub, dim, 12, neg, 1e-4), idx, dist, _spread(init, dim), 12, (1,) * 6)
-    assert "pool" not in layout["kernel"]
+    assert kernel in layout["kernel"]
     assert np.abs(got[:, 1:-1]).max(initial=0.0) == 0.0
     assert np.abs(got[:, [0, -1]] - want).max() <= 1e-4

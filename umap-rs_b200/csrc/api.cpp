@@ -2233,9 +2233,7 @@ int umap_optimizer_layout_flags(const umap_optimizer* opt, uint32_t* flags) {
   *flags = (opt->layout.lane_major ? UMAP_LAYOUT_LANE_MAJOR : 0u) |
            (opt->layout.kernel == EpochKernel::Dram ? UMAP_LAYOUT_DRAM | UMAP_LAYOUT_TWELVE_NEGATIVES : 0u) |
            (opt->layout.kernel == EpochKernel::Pool ? UMAP_LAYOUT_POOLED : 0u) |
-           (opt->layout.kernel == EpochKernel::Group4 ? UMAP_LAYOUT_GROUP_4 : 0u) |
-           (opt->layout.kernel == EpochKernel::Group8 ? UMAP_LAYOUT_GROUP_8 : 0u) |
-           (opt->layout.kernel == EpochKernel::Columns ? UMAP_LAYOUT_COLUMNS : 0u) |
+           (opt->layout.kernel == EpochKernel::Rows ? UMAP_LAYOUT_ROWS : 0u) |
            (opt->layout.order.p ? UMAP_LAYOUT_RENAMED : 0u) |
            (opt->metric_type == UMAP_METRIC_GENERIC ? UMAP_LAYOUT_GENERIC_RULE : 0u) |
            (opt->layout.task_order == TaskOrder::LengthRate ? UMAP_LAYOUT_RATE_ORDER : 0u) |

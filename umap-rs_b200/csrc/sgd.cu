@@ -418,18 +418,6 @@ __global__ void __launch_bounds__(256, MINB_DRAM) sgd_epoch_dram(
   }
 }
 
-// A firing's rows as the grouped kernels fetch them: slots 0..6 are its first seven negatives, slot 7
-// its tail.  At the default negative_sample_rate of 5 most firings draw 4 to 7 negatives (up to 10
-// where an edge that fires almost every epoch skips one; those past the slots are read one by one.
-// 16 slots measured 5% slower).
-constexpr int SLOTS = 8, NEG_SLOTS = SLOTS - 1, TAIL_SLOT = SLOTS - 1;
-
-// Negative q of the firing whose generator is `rng`.
-__device__ __forceinline__ uint32_t negative_row(const NegRng& rng, uint32_t q, uint32_t seg_lo, uint32_t seg_n) {
-  const uint64_t rnd = rng.pair(q >> 1);
-  return seg_lo + __umulhi((q & 1) ? (uint32_t)(rnd >> 32) : (uint32_t)rnd, seg_n);
-}
-
 // The epoch of L2-resident layouts: a block of POOL_BT threads takes as many tasks.  For every
 // window of 32 entries it (1) evaluates the schedule of all its tasks' entries, 8 lanes reading 64
 // consecutive bytes of a task, which leaves one bit per entry, (2) sorts the tasks that fire by
@@ -441,6 +429,12 @@ __device__ __forceinline__ uint32_t negative_row(const NegRng& rng, uint32_t q, 
 // per-lane windows cost a quarter more requests: 2M points 537 -> 474 us per epoch, 300k 102 -> 92,
 // 70k 39 -> 34.  Larger pools (256 or 512 tasks, warps taking 32 at a time from the sorted list)
 // were slower: a block's heavy warps outlast the others, 727 / 945 us at 2M.
+// Small graphs are bound by the chain of one task's firings - row loads, then 6 dependent updates -
+// with the chip half empty.  Drawing a firing's rows during the loads of the one before took the
+// generator out of it (500 points 18.6 -> 14.3 us per epoch, 10k 21.3 -> 17.5, 70k 31.0 -> 28.4, 2M
+// 456 -> 439; a lane per task: 27, 33, 40, 630).  Loading the rows themselves one firing ahead, with
+// 8 lanes per task, ran 500 points in 11 us and no larger set faster than this, but its updates
+// see older rows, and layouts of some thousand points moved by more than two runs differ.
 // `early` lets the next epoch's blocks start as soon as this launch's last ones have, otherwise at
 // its end (see sgd_epoch).
 constexpr int POOL_WIN = 32;
@@ -540,16 +534,81 @@ __global__ void __launch_bounds__(POOL_BT, MINB_POOL) sgd_epoch_pool(
       load_row<DIM>(cur, hrow);
 #pragma unroll
       for (int d = 0; d < DIM; ++d) start[d] = cur[d];
-      while (m) {
-        const uint2 en = nx;
-        const uint64_t idx = first + e;
-        m &= m - 1;
-        if (m) {
-          e = (uint32_t)__ffs(m) - 1;
-          nx = __ldg(lent + e);
+      if constexpr (GEN) {
+        while (m) {
+          const uint2 en = nx;
+          const uint64_t idx = first + e;
+          m &= m - 1;
+          if (m) {
+            e = (uint32_t)__ffs(m) - 1;
+            nx = __ldg(lent + e);
+          }
+          fired_edge<DIM, GEN, NB_POOL>(cur, row, en.x, negatives_at(epoch, en.y, p.neg_rate), snap, p, alpha, idx,
+                                        epoch, seg_lo, seg_n);
         }
-        fired_edge<DIM, GEN, NB_POOL>(cur, row, en.x, negatives_at(epoch, en.y, p.neg_rate), snap, p, alpha, idx, epoch,
-                                      seg_lo, seg_n);
+      } else {
+        // A firing's row loads are issued, then the next one's rows are drawn while they are in flight.
+        constexpr bool FAR = DIM <= 2;  // the entry after that is loaded then too (wider rows would spill)
+        uint32_t kk[NB_POOL], nneg, tail;
+        uint64_t idx;
+        auto draw = [&]() {  // rows of the firing of entry nx (the head itself: no row)
+          idx = first + e;
+          tail = nx.x;
+          nneg = negatives_at(epoch, nx.y, p.neg_rate);
+          const NegRng rng(p.seed, idx, epoch);
+          uint64_t rnd = 0;
+#pragma unroll
+          for (int q = 0; q < NB_POOL; ++q) {
+            if ((q & 1) == 0 && (q < 6 || (uint32_t)q < nneg)) rnd = rng.pair(q >> 1);
+            kk[q] = (uint32_t)q < nneg ? seg_lo + __umulhi((q & 1) ? (uint32_t)(rnd >> 32) : (uint32_t)rnd, seg_n) : row;
+          }
+        };
+        auto step = [&]() {
+          m &= m - 1;
+          if (m) {
+            e = (uint32_t)__ffs(m) - 1;
+            nx = __ldg(lent + e);
+          }
+        };
+        draw();
+        if constexpr (FAR) step();
+        for (bool more = true; more;) {
+          float o[DIM], ob[NB_POOL][DIM], g[DIM];
+          float* oth = snap + (uint64_t)tail * DIM;
+          load_row<DIM>(o, oth);
+          uint32_t ok = 0;
+#pragma unroll
+          for (int q = 0; q < NB_POOL; ++q)
+            if (kk[q] != row) {
+              ok |= 1u << q;
+              // uniform rows, rarely reused by this SM: cached in L2 only (see fired_edge)
+              if constexpr (DIM == 2) load_row_l2<DIM>(ob[q], snap + (uint64_t)kk[q] * DIM);
+              else load_row<DIM>(ob[q], snap + (uint64_t)kk[q] * DIM);
+            }
+          const uint32_t drawn = nneg;
+          const uint64_t at = idx;
+          if constexpr (!FAR) step();
+          more = m != 0;
+          if (more) {
+            draw();
+            if constexpr (FAR) step();
+          }
+          attract<DIM>(cur, o, g, p, alpha);
+#pragma unroll
+          for (int d = 0; d < DIM; ++d) cur[d] += g[d];
+          sub_row<DIM>(oth, g);
+#pragma unroll
+          for (int q = 0; q < NB_POOL; ++q)
+            if ((ok >> q) & 1u) repel<DIM>(cur, ob[q], true, p, alpha);
+          const NegRng rng(p.seed, at, epoch);
+          for (uint32_t q = NB_POOL; q < drawn; ++q) {  // more negatives than fetched together
+            const uint64_t rnd = rng.pair(q >> 1);
+            const uint32_t k = seg_lo + __umulhi((q & 1) ? (uint32_t)(rnd >> 32) : (uint32_t)rnd, seg_n);
+            if (k == row) continue;
+            load_row_l2<DIM>(o, snap + (uint64_t)k * DIM);
+            repel<DIM>(cur, o, true, p, alpha);
+          }
+        }
       }
       if ((s_split[sl] >> tl) & 1u) {
 #pragma unroll
@@ -563,7 +622,8 @@ __global__ void __launch_bounds__(POOL_BT, MINB_POOL) sgd_epoch_pool(
   if (!early) umma::grid_release();
 }
 
-// More than 128 columns: same algorithm, a thread per task, head row in global memory (owned by this
+// 8 columns or more (and 5 or more with the generic-metric rule): same algorithm, a thread per task,
+// head row in global memory (owned by this
 // lane for whole-row tasks; split tasks accumulate their delta in place with atomics).  GEN
 // selects the generic-metric rule as in fired_edge.
 template <bool GEN>
@@ -640,360 +700,103 @@ __global__ void __launch_bounds__(256) sgd_epoch_anydim(
   }
 }
 
-// ------------------------------------------------------------------------------ grouped epochs
-// Entries whose schedule a group of G lanes evaluates together (one per lane and step).
-constexpr int group_window(int g) { return g > 16 ? g : 16; }
-
-
-// What a lane knows of its group's task, and the group's current window of entries.
-template <int G>
-struct GroupTask {
-  uint32_t gl, gshift, lt, tl, r, width, seg_lo, seg_n;
-  uint64_t base;
-  bool active, split;
-
-  __device__ __forceinline__ GroupTask(const uint64_t* slice_base, const uint32_t* slice_width,
-                                       const uint32_t* split_mask, const uint32_t* rowid, const SgdParams& p,
-                                       uint64_t slice, uint64_t task) {
-    const uint32_t lane = threadIdx.x & 31;
-    gl = lane & (G - 1);
-    gshift = lane & ~(uint32_t)(G - 1);
-    lt = threadIdx.x / G;
-    tl = (uint32_t)(task & 31);
-    r = rowid[task];
-    active = r != PAD_ROW;
-    width = slice_width[slice];
-    base = slice_base[slice];
-    split = (split_mask[slice] >> tl) & 1u;
-    seg_lo = 0;
-    seg_n = p.n_vertices;
-    if (p.row_seg && active) {
-      const uint32_t sg = p.row_seg[r];
-      seg_lo = (uint32_t)p.seg_off[sg];
-      seg_n = (uint32_t)(p.seg_off[sg + 1] - p.seg_off[sg]);
-    }
-  }
-  __device__ __forceinline__ uint64_t entry_index(uint32_t e) const { return base + (uint64_t)tl * width + e; }
-  // Fires of the window [ew, ew + group_window(G)): returns their mask and lists {tail, negatives} in
-  // `fire`, in entry order.
-  __device__ __forceinline__ uint32_t window(const uint2* __restrict__ entry, uint32_t ew,
-                                             uint32_t epoch, uint32_t neg_rate, uint2* fire) const {
-    constexpr int EPL = group_window(G) / G;
-    uint2 en[EPL];
-#pragma unroll
-    for (int i = 0; i < EPL; ++i) {
-      const uint32_t e = ew + i * G + gl;
-      en[i] = active && e < width ? __ldg(entry + entry_index(e)) : make_uint2(0u, 0u);
-    }
-    uint32_t m = 0;
-#pragma unroll
-    for (int i = 0; i < EPL; ++i) {
-      const bool f = fires_at(epoch, en[i].y);
-      const uint32_t b = (__ballot_sync(0xFFFFFFFFu, f) >> gshift) & (G == 32 ? 0xFFFFFFFFu : (1u << (G & 31)) - 1u);
-      if (f) fire[__popc(m) + __popc(b & ((1u << gl) - 1u))] = make_uint2(en[i].x, negatives_at(epoch, en[i].y, neg_rate));
-      m |= b << (i * G);
-    }
-    return m;
-  }
-};
-
-// Small graphs (1-D and 2-D to 4-D rows): G lanes per task.  sgd_epoch_kernel2 leaves such a
-// graph bound by one lane's chain - schedule, generator, row loads and the sequential row updates
-// of 10 or so firings one after another, its warp's other lanes diverged - with most of the chip
-// idle (500 points: 27 us per epoch, 32 warps).  Here the lanes of a group evaluate the schedule
-// of 16 entries together, each fetches SLOTS / G of a firing's row slots, one firing ahead of the
-// arithmetic, and all of them apply the updates of the head row, redundantly, with the rows
-// exchanged by shuffles; only the chain of row updates is left.  The warp's 32 / G tasks are
-// neighbours of the layout's order, so they fire about equally often.
-// The draws are those of sgd_epoch_kernel2 (same entry index, epoch and pair).  Rows are read
-// through L2: a launch overlaps the previous epoch's end up to grid_wait, and the schedule of a
-// task's first window, which does not depend on the embedding, is evaluated before it.
-template <int DIM, int G>
-__global__ void __launch_bounds__(256) sgd_epoch_group(
+// Rows of 5 to 7 columns: a thread per task with its head row in registers, a firing's tail and
+// negative rows fetched together, the warp's lanes at the same entry.  A task that is a part of a
+// row adds each move to the live row and reads it back, so that the parts of a row move together;
+// one merge per firing runs twice as fast (48 us), but by then the layouts differ from one another
+// by up to eight times as much as two runs do.  sgd_epoch_anydim, which keeps the head row in global memory, pays a
+// dependent round trip per column instead (20k points, 5-D: 515 us per epoch, here 106; 3,000: 396,
+// here 93).  What is left is the chain of read-backs of the partial rows.
+template <int DIM>
+__global__ void __launch_bounds__(256) sgd_epoch_rows(
     const uint64_t* __restrict__ slice_base, const uint32_t* __restrict__ slice_width,
     const uint32_t* __restrict__ split_mask, const uint32_t* __restrict__ rowid,
     const uint2* __restrict__ entry, uint64_t n_slices, float* __restrict__ live, float* snap,
     SgdParams p, uint32_t epoch, float alpha) {
-  constexpr int R = SLOTS / G;  // row slots per lane: slot s belongs to lane s / R
-  __shared__ uint2 s_fire[256 / G][group_window(G) + 1];
-  umma::grid_release();
-  const uint64_t task = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) / G;
-  const uint64_t slice = task >> 5;  // the same for a whole warp
+  constexpr int NB = 6;  // negative rows fetched together
+  const uint64_t slice = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const uint32_t lane = threadIdx.x & 31;
   if (slice >= n_slices) return;
-  const GroupTask<G> t(slice_base, slice_width, split_mask, rowid, p, slice, task);
-  uint2* fire = s_fire[t.lt];
-  uint32_t m = t.window(entry, 0, epoch, p.neg_rate, fire);
-  umma::grid_wait();
-  float cur[DIM], start[DIM];
-  float* hrow = live + (uint64_t)(t.active ? t.r : 0) * DIM;
-  load_row_l2<DIM>(cur, hrow);
+  const uint32_t r = rowid[slice * 32 + lane];
+  if (r == PAD_ROW) return;
+  const uint32_t width = slice_width[slice];
+  const uint64_t first = slice_base[slice] + (uint64_t)lane * width;
+  const bool split = (split_mask[slice] >> lane) & 1u;
+  uint32_t seg_lo = 0, seg_n = p.n_vertices;
+  if (p.row_seg) {
+    const uint32_t sg = p.row_seg[r];
+    seg_lo = (uint32_t)p.seg_off[sg];
+    seg_n = (uint32_t)(p.seg_off[sg + 1] - p.seg_off[sg]);
+  }
+  float* hrow = live + (uint64_t)r * DIM;
+  float cur[DIM];
+  load_row<DIM>(cur, hrow);
+  auto move = [&](const float (&g)[DIM]) {
 #pragma unroll
-  for (int d = 0; d < DIM; ++d) start[d] = cur[d];
-
-  float x[R][DIM];       // this lane's slots of the firing at hand
-  uint32_t kk[R];
-  bool ok[R];
-  uint32_t nneg = 0;
-  uint64_t idx = 0;
-  // slots of firing f (of `count`) of the window at ew; `left` holds the window's fires from f on
-  auto fetch = [&](uint32_t f, uint32_t count, uint32_t ew, uint32_t& left, float (&nx)[R][DIM], uint32_t (&nk)[R],
-                   bool (&nok)[R], uint32_t& nn, uint64_t& ni) {
-    const bool has = f < count;
-    const uint2 fe = has ? fire[f] : make_uint2(0u, 0u);
-    nn = fe.y;
-    ni = t.entry_index(ew + (left ? __ffs(left) - 1 : 0));
-    left &= left - 1;
-    const NegRng rng(p.seed, ni, epoch);
-    uint64_t rnd = 0;
-#pragma unroll
-    for (int i = 0; i < R; ++i) {
-      const uint32_t s = t.gl * R + i;
-      if (i == 0 || (i & 1) == 0) rnd = rng.pair(s >> 1);
-      const uint32_t rv = (s & 1) ? (uint32_t)(rnd >> 32) : (uint32_t)rnd;
-      nk[i] = s == TAIL_SLOT ? fe.x : t.seg_lo + __umulhi(rv, t.seg_n);
-      const bool want = has && (s == TAIL_SLOT || s < nn);
-      nok[i] = want && (s == TAIL_SLOT || nk[i] != t.r);
-      if (want) load_row_l2<DIM>(nx[i], snap + (uint64_t)nk[i] * DIM);
-      else
-#pragma unroll
-        for (int d = 0; d < DIM; ++d) nx[i][d] = 0.0f;
+    for (int d = 0; d < DIM; ++d) {
+      cur[d] += g[d];
+      if (split) atomicAdd(hrow + d, g[d]);
     }
   };
-  for (uint32_t ew = 0;;) {
-    __syncwarp();
-    const uint32_t count = (uint32_t)__popc(m);
-    const uint32_t rounds = __reduce_max_sync(0xFFFFFFFFu, count);
-    uint32_t left = m;
-    if (rounds) fetch(0, count, ew, left, x, kk, ok, nneg, idx);
-    for (uint32_t f = 0; f < rounds; ++f) {
-      float nx[R][DIM];
-      uint32_t nk[R], nn = 0;
-      bool nok[R];
-      uint64_t ni = 0;
-      if (f + 1 < rounds) fetch(f + 1, count, ew, left, nx, nk, nok, nn, ni);
-      const bool has = f < count;
+  for (uint32_t ew = 0; ew < width; ew += 4) {  // width is a multiple of 4 (slice_meta_kernel)
+    uint2 win[4];
+#pragma unroll
+    for (int j = 0; j < 4; j += 2) {
+      const uint4 v = __ldg(reinterpret_cast<const uint4*>(entry + first + ew + j));
+      win[j] = make_uint2(v.x, v.y);
+      win[j + 1] = make_uint2(v.z, v.w);
+    }
+#pragma unroll 1
+    for (uint32_t j = 0; j < 4; ++j) {
+      const uint2 en = j == 0 ? win[0] : j == 1 ? win[1] : j == 2 ? win[2] : win[3];
+      if (!fires_at(epoch, en.y)) continue;
+      float* oth = snap + (uint64_t)en.x * DIM;
+      const uint32_t nneg = negatives_at(epoch, en.y, p.neg_rate);
+      const NegRng rng(p.seed, first + ew + j, epoch);
+      float o[DIM], g[DIM], df[DIM], x[NB][DIM];
+      uint32_t kk[NB];
+      if (split) load_row_l2<DIM>(cur, hrow);
+      load_row<DIM>(o, oth);
+      auto fetch = [&](uint32_t q0) {  // negatives q0 .. q0 + NB - 1 (the head itself: none)
+        uint64_t rnd = 0;
+#pragma unroll
+        for (int q = 0; q < NB; ++q) {
+          if ((q & 1) == 0) rnd = rng.pair((q0 + q) >> 1);
+          kk[q] = q0 + q < nneg ? seg_lo + __umulhi((q & 1) ? (uint32_t)(rnd >> 32) : (uint32_t)rnd, seg_n) : r;
+          if (kk[q] != r) load_row<DIM>(x[q], snap + (uint64_t)kk[q] * DIM);
+        }
+      };
+      fetch(0);
       // attractive step (optimize_layout_euclidean.rs:284-306)
       {
-        float o[DIM], g[DIM];
+        float num, inv;
 #pragma unroll
-        for (int d = 0; d < DIM; ++d) o[d] = __shfl_sync(0xFFFFFFFFu, x[R - 1][d], G - 1, G);
-        attract<DIM>(cur, o, g, p, alpha);
-        if (has) {
+        for (int d = 0; d < DIM; ++d) df[d] = cur[d] - o[d];
+        attract_terms(square_ftz<DIM>(df), p, num, inv);
 #pragma unroll
-          for (int d = 0; d < DIM; ++d) cur[d] += g[d];
-          if (t.gl == G - 1) sub_row<DIM>(snap + (uint64_t)kk[R - 1] * DIM, g);
-        }
+        for (int d = 0; d < DIM; ++d) g[d] = clip4((num * df[d]) * inv) * alpha;
+        move(g);
+        sub_row<DIM>(oth, g);
       }
       // negative samples (:313-341)
-      unsigned okb[R];
+      for (uint32_t q0 = 0; q0 < nneg; q0 += NB) {
+        if (q0 > 0) fetch(q0);
 #pragma unroll
-      for (int i = 0; i < R; ++i) okb[i] = __ballot_sync(0xFFFFFFFFu, ok[i]) >> t.gshift;
-      const uint32_t nmax = __reduce_max_sync(0xFFFFFFFFu, nneg);
+        for (int q = 0; q < NB; ++q) {
+          if (kk[q] == r) continue;
+          if (split) load_row_l2<DIM>(cur, hrow);
 #pragma unroll
-      for (int q = 0; q < NEG_SLOTS; ++q) {
-        if ((uint32_t)q >= nmax) break;
-        float o[DIM];
+          for (int d = 0; d < DIM; ++d) df[d] = cur[d] - x[q][d];
+          const float ds = square_ftz<DIM>(df), inv = repel_inv(ds, p);
+          if (!(ds > 0.0f)) continue;  // a NaN distance (a NaN row) moves nothing
 #pragma unroll
-        for (int d = 0; d < DIM; ++d) o[d] = __shfl_sync(0xFFFFFFFFu, x[q % R][d], q / R, G);
-        repel<DIM>(cur, o, (okb[q % R] >> (q / R)) & 1u, p, alpha);
-      }
-      for (uint32_t q = NEG_SLOTS; q < nmax; ++q) {  // more negatives than slots: one at a time
-        float o[DIM];
-        const uint32_t k = negative_row(NegRng(p.seed, idx, epoch), q, t.seg_lo, t.seg_n);
-        const bool apply = q < nneg && k != t.r;
-        if (apply) load_row_l2<DIM>(o, snap + (uint64_t)k * DIM);
-        else
-#pragma unroll
-          for (int d = 0; d < DIM; ++d) o[d] = 0.0f;
-        repel<DIM>(cur, o, apply, p, alpha);
-      }
-#pragma unroll
-      for (int i = 0; i < R; ++i) {
-#pragma unroll
-        for (int d = 0; d < DIM; ++d) x[i][d] = nx[i][d];
-        kk[i] = nk[i];
-        ok[i] = nok[i];
-      }
-      nneg = nn;
-      idx = ni;
-    }
-    ew += group_window(G);
-    if (ew >= t.width) break;
-    __syncwarp();
-    m = t.window(entry, ew, epoch, p.neg_rate, fire);
-  }
-  if (t.active && t.gl == 0) {
-    if (t.split) {
-#pragma unroll
-      for (int d = 0; d < DIM; ++d) atomicAdd(hrow + d, cur[d] - start[d]);
-    } else {
-      store_row<DIM>(hrow, cur);
-    }
-  }
-}
-
-// Rows of more than 4 columns (n_components 5 to 128): a group of G lanes per task, lane j holding
-// columns j, j + G, ... (C of them) of the head row in registers, so a row is one coalesced read and
-// a squared distance one shuffle reduction.  The schedule, the generator (lane q draws negative q)
-// and the fetch of a firing's rows one firing ahead are those of sgd_epoch_group.  A thread per task
-// with its head row in global memory (sgd_epoch_anydim) pays a dependent global round trip for
-// every column of every update.
-template <int G, int C, bool GEN>
-__global__ void __launch_bounds__(256) sgd_epoch_columns(
-    const uint64_t* __restrict__ slice_base, const uint32_t* __restrict__ slice_width,
-    const uint32_t* __restrict__ split_mask, const uint32_t* __restrict__ rowid,
-    const uint2* __restrict__ entry, uint64_t n_slices, float* __restrict__ live, float* snap,
-    SgdParams p, uint32_t epoch, float alpha) {
-  constexpr int NS = 8;  // rows fetched ahead: the first 7 negatives and the tail
-  __shared__ uint2 s_fire[256 / G][group_window(G) + 1];
-  umma::grid_release();
-  const uint64_t task = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) / G;
-  const uint64_t slice = task >> 5;
-  if (slice >= n_slices) return;
-  const GroupTask<G> t(slice_base, slice_width, split_mask, rowid, p, slice, task);
-  uint2* fire = s_fire[t.lt];
-  uint32_t m = t.window(entry, 0, epoch, p.neg_rate, fire);
-  umma::grid_wait();
-  const uint32_t dim = p.dim;
-  float cur[C], start[C];
-  float* hrow = live + (uint64_t)(t.active ? t.r : 0) * dim;
-  // this lane's columns of a row (0 where there is none)
-  auto load = [&](float (&v)[C], const float* row, bool want) {
-#pragma unroll
-    for (int i = 0; i < C; ++i) {
-      const uint32_t c = t.gl + i * G;
-      v[i] = want && c < dim ? __ldcg(row + c) : 0.0f;
-    }
-  };
-  load(cur, hrow, t.active);
-#pragma unroll
-  for (int i = 0; i < C; ++i) start[i] = cur[i];
-
-  auto square = [&](const float (&df)[C]) {
-    float ds = t.gl == 0 ? 1.17549435e-38f : 0.0f;  // as in square_ftz
-#pragma unroll
-    for (int i = 0; i < C; ++i) ds = fmaf(df[i], df[i], ds);
-#pragma unroll
-    for (int o = G / 2; o > 0; o >>= 1) ds += __shfl_xor_sync(0xFFFFFFFFu, ds, o);
-    return ds;
-  };
-  auto repel = [&](const float (&o)[C], bool apply) {
-    float df[C];
-#pragma unroll
-    for (int i = 0; i < C; ++i) df[i] = cur[i] - o[i];
-    const float ds = square(df);
-    if constexpr (GEN) {
-      float den;
-      const float gr = metric_coeff(ds, p.a, p.two_b, p.pos_rep, 0.0f, &den);
-      if (apply) {
-#pragma unroll
-        for (int i = 0; i < C; ++i) cur[i] += clip4(gr * __fdividef(df[i], den)) * alpha;
-      }
-    } else {
-      const float inv = repel_inv(ds, p);
-      if (apply && ds > 0.0f) {
-#pragma unroll
-        for (int i = 0; i < C; ++i) cur[i] = fmaf(clip4((p.pos_rep * df[i]) * inv), alpha, cur[i]);
-      }
-    }
-  };
-  float x[NS][C];
-  uint32_t kk = 0, nneg = 0;
-  uint64_t idx = 0;
-  auto fetch = [&](uint32_t f, uint32_t count, uint32_t ew, uint32_t& left, float (&nx)[NS][C], uint32_t& nk,
-                   uint32_t& nn, uint64_t& ni) {
-    const bool has = f < count;
-    const uint2 fe = has ? fire[f] : make_uint2(0u, 0u);
-    nn = fe.y;
-    ni = t.entry_index(ew + (left ? __ffs(left) - 1 : 0));
-    left &= left - 1;
-    nk = t.gl == NS - 1 ? fe.x : negative_row(NegRng(p.seed, ni, epoch), t.gl, t.seg_lo, t.seg_n);
-#pragma unroll
-    for (int s = 0; s < NS; ++s) {
-      const uint32_t k = __shfl_sync(0xFFFFFFFFu, nk, s, G);
-      load(nx[s], snap + (uint64_t)k * dim, has && (s == NS - 1 || (uint32_t)s < nn));
-    }
-  };
-
-  for (uint32_t ew = 0;;) {
-    __syncwarp();
-    const uint32_t count = (uint32_t)__popc(m);
-    const uint32_t rounds = __reduce_max_sync(0xFFFFFFFFu, count);
-    uint32_t left = m;
-    if (rounds) fetch(0, count, ew, left, x, kk, nneg, idx);
-    for (uint32_t f = 0; f < rounds; ++f) {
-      float nx[NS][C];
-      uint32_t nk = 0, nn = 0;
-      uint64_t ni = 0;
-      if (f + 1 < rounds) fetch(f + 1, count, ew, left, nx, nk, nn, ni);
-      const bool has = f < count;
-      {
-        float df[C];
-#pragma unroll
-        for (int i = 0; i < C; ++i) df[i] = cur[i] - x[NS - 1][i];
-        const float ds = square(df);
-        float gc, inv;
-        if constexpr (GEN) {
-          float den;
-          gc = metric_coeff(ds, p.a, p.two_b, p.two_b, -1.0f, &den);
-          inv = __fdividef(1.0f, den);
-        } else {
-          attract_terms(ds, p, gc, inv);
-        }
-        const uint32_t k = __shfl_sync(0xFFFFFFFFu, kk, NS - 1, G);
-        if (has) {
-#pragma unroll
-          for (int i = 0; i < C; ++i) {
-            const float g = clip4((gc * df[i]) * inv) * alpha;
-            cur[i] += g;
-            const uint32_t c = t.gl + i * G;
-            if (c < dim) atomicAdd(snap + (uint64_t)k * dim + c, -g);
-          }
+          for (int d = 0; d < DIM; ++d) g[d] = clip4((p.pos_rep * df[d]) * inv) * alpha;
+          move(g);
         }
       }
-      const uint32_t nmax = __reduce_max_sync(0xFFFFFFFFu, nneg);
-      const unsigned okb = __ballot_sync(0xFFFFFFFFu, t.gl < NS - 1 && t.gl < nneg && kk != t.r) >> t.gshift;
-#pragma unroll
-      for (int q = 0; q < NS - 1; ++q) {
-        if ((uint32_t)q >= nmax) break;
-        repel(x[q], (okb >> q) & 1u);
-      }
-      for (uint32_t q = NS - 1; q < nmax; ++q) {
-        float o[C];
-        const uint32_t k = negative_row(NegRng(p.seed, idx, epoch), q, t.seg_lo, t.seg_n);
-        const bool apply = q < nneg && k != t.r;
-        load(o, snap + (uint64_t)k * dim, apply);
-        repel(o, apply);
-      }
-      if (t.split && has) {  // a partial row: merge this firing's moves with the other parts' so far
-#pragma unroll
-        for (int i = 0; i < C; ++i) {
-          const uint32_t c = t.gl + i * G;
-          if (c >= dim) continue;
-          const float moved = cur[i] - start[i];
-          cur[i] = start[i] = atomicAdd(hrow + c, moved) + moved;
-        }
-      }
-#pragma unroll
-      for (int s = 0; s < NS; ++s)
-#pragma unroll
-        for (int i = 0; i < C; ++i) x[s][i] = nx[s][i];
-      kk = nk;
-      nneg = nn;
-      idx = ni;
-    }
-    ew += group_window(G);
-    if (ew >= t.width) break;
-    __syncwarp();
-    m = t.window(entry, ew, epoch, p.neg_rate, fire);
-  }
-  if (t.active) {
-#pragma unroll
-    for (int i = 0; i < C; ++i) {
-      const uint32_t c = t.gl + i * G;
-      if (c < dim && !t.split) hrow[c] = cur[i];
     }
   }
+  if (!split) store_row<DIM>(hrow, cur);
 }
 
 // ------------------------------------------------------------------------------ K5 pieces
@@ -1406,35 +1209,26 @@ bool small_graph(uint64_t n_slices) {
 }
 
 // The epoch kernel of a layout.
-//  * Columns / AnyDim: rows of 5 to 128 and of more columns.
+//  * Rows / AnyDim: rows of 5 to 7 and of more columns.  Forces of 8-D layouts and up are so small
+//    that the order of the updates, which every faster kernel changes, shows in the result: 30k
+//    points in 8-D differ between the two kernels by 2e-4 of their size, between two runs of AnyDim
+//    by 4e-5 (6-D: 2e-4 and 6e-5, 5-D: 2.4e-4 and 9e-5).
 //  * Dram: renamed 1-D and 2-D layouts whose snapshot (4 * dim bytes per vertex) is above 80 MB, so
 //    that with the edge stream it does not stay in the 126 MB L2.  The random rows then cost DRAM
 //    bursts, and the interleaved order's whole 256-byte rows per warp use them better than a task's
 //    contiguous entries (2-D rolls, 30 epochs, Dram interleaved against Pool lane major, ms: 5M points
 //    34.7 / 28.2, 8M 55.1 / 44.6, 12M 94.6 / 98.7, 16M 149.6 / 156.9, 20M 207.2 / 221.6).
-//  * Group8 / Group4: G lanes per task while T tasks of G lanes are at most about 1,450 threads per
-//    SM (2-D mixtures, k = 15, us per epoch, Group8 / Group4 / Pool: 500 points 12.2 / 13.9 / 19.9,
-//    10k 18.5 / 22.7 / 24.3, 14k 20.2 / 22.0 / 24.6, 22k 26.7 / 22.7 / 26.1, 30k 34.0 / 27.4 / 27.6,
-//    70k 70 / 47 / 34).
-//  * Pool: everything else, and the generic-metric rule at every size.
-// UMAP_B200_SGD_KERNEL=pool / group4 / group8 / dram forces one that can run the layout.
-EpochKernel pick_epoch_kernel(uint64_t n, uint32_t dim, uint64_t n_tasks, bool renamed, bool segmented, bool generic) {
-  if (dim > 128) return EpochKernel::AnyDim;
-  if (dim > 4) return EpochKernel::Columns;
+//  * Pool: everything else.
+// UMAP_B200_SGD_KERNEL=pool / dram forces one that can run the layout.
+EpochKernel pick_epoch_kernel(uint64_t n, uint32_t dim, bool renamed, bool segmented, bool generic) {
+  if (dim > 4) return dim <= 7 && !generic ? EpochKernel::Rows : EpochKernel::AnyDim;
   const bool can_dram = dim <= 2 && !generic && !segmented;
   if (const char* e = getenv("UMAP_B200_SGD_KERNEL")) {
     if (!strcmp(e, "dram") && can_dram) return EpochKernel::Dram;
     if (!strcmp(e, "pool")) return EpochKernel::Pool;
-    if (!strcmp(e, "group4") && !generic) return EpochKernel::Group4;
-    if (!strcmp(e, "group8") && !generic) return EpochKernel::Group8;
   }
   if (can_dram && renamed && n * dim * 4 > 80000000ull) return EpochKernel::Dram;
-  if (generic) return EpochKernel::Pool;
-  int dev = 0, sms = 0;
-  UB_CUDA(cudaGetDevice(&dev));
-  UB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  const uint64_t room = 1450ull * (uint64_t)std::max(sms, 1);
-  return n_tasks * 8 <= room ? EpochKernel::Group8 : n_tasks * 4 <= room ? EpochKernel::Group4 : EpochKernel::Pool;
+  return EpochKernel::Pool;
 }
 
 // Whether a plain fit's layout renames its vertices into a locality order (order.cu): from the
@@ -1520,7 +1314,7 @@ void build_sgd_layout(const uint64_t* kept_ptr, const uint32_t* ktail, const dou
   if ((uint64_t)n_seg << len_bits >= (1ull << 32)) throw Error(UNSUPPORTED, "too many instances for the task sort key");
   const int seg_bits = n_seg ? bits_for(n_seg) : 0;
   const bool renamed = L.order.p != nullptr;
-  L.kernel = pick_epoch_kernel(n, dim, T, renamed, seg != nullptr, generic);
+  L.kernel = pick_epoch_kernel(n, dim, renamed, seg != nullptr, generic);
   L.lane_major = L.kernel != EpochKernel::Dram;
   TaskOrder torder = pick_task_order(renamed, small_graph((T + 31) / 32), seg != nullptr);
   if (torder == TaskOrder::LengthRate && len_bits + seg_bits + RATE_BITS > 32) torder = TaskOrder::Length;
@@ -1633,11 +1427,10 @@ void launch_epoch(void (*k)(P...), unsigned grid, unsigned bt, bool overlap, cud
   count_launch();
 }
 
-// The launch may overlap the end of the epoch before it (`overlap`): every kernel but Dram and AnyDim
-// evaluates its schedule before grid_wait.  A small launch is released to the next one when its
-// blocks start - the next epoch's blocks find free slots - and so is a large one (2M points: 474
-// against 484 us per epoch); the pooled kernel in between releases at its blocks' end, since the next
-// epoch's early blocks would fill the SMs unevenly (70k points: 34 against 41 us).
+// The launch may overlap the end of the epoch before it (`overlap`): the pooled kernel evaluates its
+// schedule before grid_wait.  A large launch is released to the next one when its last blocks start
+// (2M points: 474 against 484 us per epoch), a smaller one at its blocks' end, since the next epoch's
+// early blocks would fill the SMs unevenly (20k points: 19.2 against 28.6 us, 70k: 34 against 41).
 void sgd_epoch(const SgdLayout& L, float* live, float* snap, const SgdParams& p, uint32_t epoch, float alpha,
                bool overlap, cudaStream_t s) {
   if (L.n_slices == 0) return;
@@ -1650,37 +1443,21 @@ void sgd_epoch(const SgdLayout& L, float* live, float* snap, const SgdParams& p,
   };
 #define UB_SGD_ARGS L.slice_base.p, L.slice_width.p, L.split_mask.p, L.rowid.p, L.entry.p, L.n_slices, live, snap, \
                     p, epoch, alpha
-  auto grouped = [&](auto k, uint32_t lanes) { launch_epoch(k, blocks(tasks * lanes, BT), BT, overlap, s, UB_SGD_ARGS); };
   auto pooled = [&](auto k) {
     const unsigned g = blocks(tasks, POOL_BT);
     launch_epoch(k, g, POOL_BT, overlap, s, UB_SGD_ARGS, g > 8000u);
   };
   const bool gen = p.generic_metric;
   switch (L.kernel) {
-    case EpochKernel::Group8:
-      if (p.dim == 1) grouped(sgd_epoch_group<1, 8>, 8);
-      else if (p.dim == 2) grouped(sgd_epoch_group<2, 8>, 8);
-      else if (p.dim == 3) grouped(sgd_epoch_group<3, 8>, 8);
-      else grouped(sgd_epoch_group<4, 8>, 8);
-      break;
-    case EpochKernel::Group4:
-      if (p.dim == 1) grouped(sgd_epoch_group<1, 4>, 4);
-      else if (p.dim == 2) grouped(sgd_epoch_group<2, 4>, 4);
-      else if (p.dim == 3) grouped(sgd_epoch_group<3, 4>, 4);
-      else grouped(sgd_epoch_group<4, 4>, 4);
-      break;
     case EpochKernel::Pool:
       if (p.dim == 1) gen ? pooled(sgd_epoch_pool<1, true>) : pooled(sgd_epoch_pool<1, false>);
       else if (p.dim == 2) gen ? pooled(sgd_epoch_pool<2, true>) : pooled(sgd_epoch_pool<2, false>);
       else if (p.dim == 3) gen ? pooled(sgd_epoch_pool<3, true>) : pooled(sgd_epoch_pool<3, false>);
       else gen ? pooled(sgd_epoch_pool<4, true>) : pooled(sgd_epoch_pool<4, false>);
       break;
-    case EpochKernel::Columns:
-      if (p.dim <= 8) gen ? grouped(sgd_epoch_columns<8, 1, true>, 8) : grouped(sgd_epoch_columns<8, 1, false>, 8);
-      else if (p.dim <= 16) gen ? grouped(sgd_epoch_columns<16, 1, true>, 16) : grouped(sgd_epoch_columns<16, 1, false>, 16);
-      else if (p.dim <= 32) gen ? grouped(sgd_epoch_columns<32, 1, true>, 32) : grouped(sgd_epoch_columns<32, 1, false>, 32);
-      else if (p.dim <= 64) gen ? grouped(sgd_epoch_columns<32, 2, true>, 32) : grouped(sgd_epoch_columns<32, 2, false>, 32);
-      else gen ? grouped(sgd_epoch_columns<32, 4, true>, 32) : grouped(sgd_epoch_columns<32, 4, false>, 32);
+    case EpochKernel::Rows:
+      launch_epoch(p.dim == 5 ? sgd_epoch_rows<5> : p.dim == 6 ? sgd_epoch_rows<6> : sgd_epoch_rows<7>,
+                   blocks(tasks, BT), BT, false, s, UB_SGD_ARGS);
       break;
     case EpochKernel::Dram:
       launch_epoch(p.dim == 1 ? sgd_epoch_dram<1> : sgd_epoch_dram<2>, blocks(tasks, BT), BT, false, s, UB_SGD_ARGS);

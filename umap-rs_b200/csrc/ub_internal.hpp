@@ -182,7 +182,7 @@ constexpr uint64_t MAX_EPOCHS = 1ull << 21;
 enum class TaskOrder { Length, LengthRate, RowBlock, Row };
 
 // Which kernel runs the layout's epochs (sgd.cu, pick_epoch_kernel).
-enum class EpochKernel { Pool, Group8, Group4, Columns, AnyDim, Dram };
+enum class EpochKernel { Pool, Rows, AnyDim, Dram };
 
 struct SgdLayout {
   uint64_t n_vertices = 0, n_edges = 0, n_entries = 0, n_slices = 0, n_tasks = 0;

@@ -664,17 +664,12 @@ class Optimizer(_Handle):
         _, dim = self.dims()
         eight = eight and dim <= 2 and not generic  # the generic rule keeps the 4-negatives budget
         twelve = twelve and dim <= 2 and not generic
-        nb, minb = (12, 3) if twelve else (8, 4) if eight else (4, 5)
         gen = "true" if generic else "false"
-        kernel = (f"sgd_epoch_kernel2<{dim}, {gen}, {nb}, {minb}, {'true' if lm else 'false'}>" if dim <= 4
-                  else f"sgd_epoch_anydim<{gen}>")
+        kernel = f"sgd_epoch_anydim<{gen}>"
         if f.value & bit["POOLED"]:
             kernel = f"sgd_epoch_pool<{dim}, {gen}>"
-        elif f.value & (bit["GROUP_4"] | bit["GROUP_8"]):
-            kernel = f"sgd_epoch_group<{dim}, {8 if f.value & bit['GROUP_8'] else 4}>"
-        elif f.value & bit["COLUMNS"]:
-            lanes, each = (8, 1) if dim <= 8 else (16, 1) if dim <= 16 else (32, 1 if dim <= 32 else 2 if dim <= 64 else 4)
-            kernel = f"sgd_epoch_columns<{lanes}, {each}, {gen}>"
+        elif f.value & bit["ROWS"]:
+            kernel = f"sgd_epoch_rows<{dim}>"
         elif f.value & bit["DRAM"]:
             kernel = f"sgd_epoch_dram<{dim}>"
         order = ("length+rate" if f.value & bit["RATE_ORDER"] else "row blocks" if f.value & bit["BLOCK_ORDER"]

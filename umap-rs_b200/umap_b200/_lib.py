@@ -41,8 +41,7 @@ class WarmStartParamsC(C.Structure):
 
 # umap_optimizer_layout_flags bits (UMAP_LAYOUT_* in include/umap_b200.h)
 LAYOUT_FLAGS = {"LANE_MAJOR": 1, "EIGHT_NEGATIVES": 2, "RENAMED": 4, "GENERIC_RULE": 8, "TWELVE_NEGATIVES": 16,
-                "RATE_ORDER": 32, "BLOCK_ORDER": 64, "ROW_ORDER": 128, "POOLED": 256, "GROUP_4": 512, "GROUP_8": 1024,
-                "COLUMNS": 2048, "DRAM": 4096}
+                "RATE_ORDER": 32, "BLOCK_ORDER": 64, "ROW_ORDER": 128, "POOLED": 256, "ROWS": 512, "DRAM": 1024}
 
 WARM_START_PHASES = ("prepare", "subsample_fit", "mlp_train", "mlp_predict", "wait_full_graph", "fit",
                      "full_graph_overlapped", "total")
