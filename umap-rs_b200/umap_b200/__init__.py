@@ -665,7 +665,9 @@ class Optimizer(_Handle):
         eight = eight and dim <= 2 and not generic  # the generic rule keeps the 4-negatives budget
         twelve = twelve and dim <= 2 and not generic
         gen = "true" if generic else "false"
-        kernel = f"sgd_epoch_anydim<{gen}>"
+        nb, minb = (12, 3) if twelve else (8, 4) if eight else (4, 5)
+        kernel = (f"sgd_epoch_kernel2<{dim}, {gen}, {nb}, {minb}, {'true' if lm else 'false'}>" if dim <= 4
+                  else f"sgd_epoch_anydim<{gen}>")
         if f.value & bit["POOLED"]:
             kernel = f"sgd_epoch_pool<{dim}, {gen}>"
         elif f.value & bit["ROWS"]:
