@@ -7,6 +7,7 @@
 // evaluated in double by CUDA's exp() and rounded once to f32.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 
 #include "ub_internal.hpp"
@@ -50,8 +51,12 @@ __device__ __forceinline__ void stage_rows(T* s, const T* __restrict__ g, uint64
 }
 
 // ------------------------------------------------------------------------------ K1
-// smooth_knn_dist.rs:78-186 for one row per thread.
-template <bool SMEM>
+// smooth_knn_dist.rs:78-186, L lanes per row (1, 4 or 16).  The bisection's double-precision exponentials
+// bound it: up to 64 rounds of k - 1 of them, one after another in a thread.  While the rows leave
+// threads idle, L lanes share a round's exponentials, and all of them add these up in the reference's
+// order (10k rows of 15, L = 1 / 16: 73 / 50 us; 30k of 30, L = 1 / 4: 144 / 118 us; at 70k of 15 the
+// double-precision units are full and the exchange only costs: 97 / 142 us).
+template <bool SMEM, int L>
 __global__ void __launch_bounds__(BT) smooth_knn_kernel(const float* __restrict__ dist, uint64_t n,
                                                         uint32_t k, GraphParams gp,
                                                         float* __restrict__ sigmas,
@@ -59,15 +64,19 @@ __global__ void __launch_bounds__(BT) smooth_knn_kernel(const float* __restrict_
                                                         unsigned* __restrict__ need_global) {
   extern __shared__ float s_rows[];
   const uint32_t stride = k | 1u;
-  const uint64_t row0 = (uint64_t)blockIdx.x * BT;
-  const uint32_t rows = (uint32_t)min((uint64_t)BT, n - row0);
+  constexpr uint32_t ROWS = BT / L;
+  const uint64_t row0 = (uint64_t)blockIdx.x * ROWS;
+  const uint32_t rows = (uint32_t)min((uint64_t)ROWS, n - row0);
   if (SMEM) {
     stage_rows(s_rows, dist, row0, rows, k, stride);
     __syncthreads();
   }
-  if (threadIdx.x >= rows) return;
-  const uint64_t i = row0 + threadIdx.x;
-  const float* row = SMEM ? s_rows + threadIdx.x * stride : dist + i * k;
+  const uint32_t lr = threadIdx.x / L;
+  if (lr >= rows) return;
+  const uint64_t i = row0 + lr;
+  const float* row = SMEM ? s_rows + lr * stride : dist + i * k;
+  float* terms = s_rows + (ROWS + lr) * stride;  // L > 1: the row's exponentials
+  const uint32_t part = threadIdx.x & (L - 1), lanes = L == 1 ? 0u : ((1u << L) - 1u) << (threadIdx.x & 31 & ~(L - 1));
 
   // :88-97
   uint64_t non_zero_count = 0;
@@ -111,10 +120,21 @@ __global__ void __launch_bounds__(BT) smooth_knn_kernel(const float* __restrict_
   float lo = 0.0f, hi = INFINITY, mid = 1.0f;
   for (int it = 0; it < gp.n_iter; ++it) {
     float psum = 0.0f;
-    for (uint32_t j = 1; j < k; ++j) {
-      float d = __fsub_rn(row[j], rho);
-      if (d > 0.0f) psum = __fadd_rn(psum, exp_f32(-__fdiv_rn(d, mid)));
-      else psum = __fadd_rn(psum, 1.0f);
+    if constexpr (L > 1) {
+      for (uint32_t j = 1 + part; j < k; j += L) {
+        const float d = __fsub_rn(row[j], rho), e = exp_f32(-__fdiv_rn(d, mid));
+        terms[j] = d > 0.0f ? e : 1.0f;
+      }
+      __syncwarp(lanes);
+#pragma unroll 8
+      for (uint32_t j = 1; j < k; ++j) psum = __fadd_rn(psum, terms[j]);
+      __syncwarp(lanes);
+    } else {
+      for (uint32_t j = 1; j < k; ++j) {
+        float d = __fsub_rn(row[j], rho);
+        if (d > 0.0f) psum = __fadd_rn(psum, exp_f32(-__fdiv_rn(d, mid)));
+        else psum = __fadd_rn(psum, 1.0f);
+      }
     }
     if (fabsf(__fsub_rn(psum, gp.target)) < SMOOTH_K_TOLERANCE) break;
     if (psum > gp.target) {
@@ -133,9 +153,10 @@ __global__ void __launch_bounds__(BT) smooth_knn_kernel(const float* __restrict_
     float m = nd_mean(row, k, 1);
     float lim = __fmul_rn(MIN_K_DIST_SCALE, m);
     if (sigma < lim) sigma = lim;
-  } else {
+  } else if (part == 0) {
     atomicOr(need_global, 1u);
   }
+  if (part) return;
   sigmas[i] = sigma;
   rhos[i] = rho;
 }
@@ -322,60 +343,107 @@ __global__ void segment_starts_kernel(const uint32_t* __restrict__ keys, uint64_
 }
 
 // ------------------------------------------------------------------------------ K4
-// fuzzy_simplicial_set.rs:392-552 for one output row per thread: merge-join of the sorted
-// directed row r (columns col, value A[r,col]) with the transposed row r (sources c in
-// ascending order, value A[c,r]).  Emits mix*a + mix*b + (1-2mix)*a*b (:423/:488) for
-// direct entries and mix*b (:506) for transpose-only entries, dropping zeros.
+// fuzzy_simplicial_set.rs:392-552 for one output row per group of G lanes: union of the sorted
+// directed row r (columns s_c, values A[r,c]) with the transposed row r (sources c in ascending
+// order, value A[c,r]).  Emits mix*a + mix*b + (1-2mix)*a*b (:423/:488) for direct entries and
+// mix*b (:506) for transpose-only entries, dropping zeros.
+// The random reads of A[c,r] bound it, so a lane takes an entry and all of a row's are in flight at
+// once; each entry finds its place by rank: the transposed ones by their lower bound in the direct
+// row, the direct ones by a running sum of how many transposed ones sort before them.  A thread per row merging
+// serially waited for one read after another (us per launch, before and now: 30k rows of 30
+// neighbours 254 / 35, 2M of 15 1720 / 935).
+template <int G>
 __global__ void __launch_bounds__(BT) union_kernel(
     const uint32_t* __restrict__ pcol, const float* __restrict__ pw, const uint32_t* __restrict__ cnt,
     uint32_t k, const uint64_t* __restrict__ tptr, const uint32_t* __restrict__ tvals, uint64_t n,
     float mix, float prod, uint32_t* __restrict__ out_cnt, const uint64_t* __restrict__ out_ptr,
     uint32_t* __restrict__ out_idx, float* __restrict__ out_w, bool fill) {
-  const uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  extern __shared__ uint32_t s_union[];  // per group: columns, direct values, transposed values, ranks
+  const uint32_t lane = threadIdx.x & 31, gl = lane & (G - 1), shift = lane & ~(uint32_t)(G - 1);
+  const uint32_t gmask = G == 32 ? 0xFFFFFFFFu : ((1u << (G & 31)) - 1u) << shift, below = (1u << gl) - 1u;
+  const uint64_t r = ((uint64_t)blockIdx.x * BT + threadIdx.x) / G;
   if (r >= n) return;
+  uint32_t* s_c = s_union + (threadIdx.x / G) * 4 * (k + 1);
+  float* s_a = (float*)(s_c + k + 1);
+  float* s_b = s_a + k + 1;
+  uint32_t* s_h = (uint32_t*)(s_b + k + 1);  // transpose-only entries between columns i - 1 and i
   const uint64_t abase = r * k;
   const uint32_t an = cnt[r];
-  uint64_t j = tptr[r];
-  const uint64_t jend = tptr[r + 1];
-  uint32_t i = 0, count = 0;
-  uint64_t o = fill ? out_ptr[r] : 0;
-  uint32_t ca = i < an ? pcol[abase] : 0xFFFFFFFFu;
-  uint32_t pb = 0, cb = 0xFFFFFFFFu;
-  if (j < jend) { pb = tvals[j]; cb = pb / k; }
-  while (ca != 0xFFFFFFFFu || cb != 0xFFFFFFFFu) {
-    float v;
-    uint32_t col;
-    if (ca < cb) {
-      const float a = pw[abase + i];
-      v = __fadd_rn(__fadd_rn(__fmul_rn(mix, a), __fmul_rn(mix, 0.0f)), __fmul_rn(__fmul_rn(prod, a), 0.0f));
-      col = ca;
-      ++i;
-      ca = i < an ? pcol[abase + i] : 0xFFFFFFFFu;
-    } else if (ca == cb) {
-      const float a = pw[abase + i], b = pw[pb];
-      v = __fadd_rn(__fadd_rn(__fmul_rn(mix, a), __fmul_rn(mix, b)), __fmul_rn(__fmul_rn(prod, a), b));
-      col = ca;
-      ++i;
-      ca = i < an ? pcol[abase + i] : 0xFFFFFFFFu;
-      ++j;
-      if (j < jend) { pb = tvals[j]; cb = pb / k; } else cb = 0xFFFFFFFFu;
-    } else {
-      const float b = pw[pb];
-      v = __fmul_rn(mix, b);
-      col = cb;
-      ++j;
-      if (j < jend) { pb = tvals[j]; cb = pb / k; } else cb = 0xFFFFFFFFu;
-    }
-    if (v != 0.0f) {
-      if (fill) {
-        out_idx[o] = col;
-        out_w[o] = v;
-        ++o;
-      }
-      ++count;
-    }
+  const uint64_t j0 = tptr[r], jend = tptr[r + 1];
+  for (uint32_t i = gl; i <= an; i += G) {
+    s_c[i] = i < an ? pcol[abase + i] : 0xFFFFFFFFu;
+    s_a[i] = i < an ? pw[abase + i] : 0.0f;
+    s_b[i] = 0.0f;
+    s_h[i] = 0;
   }
-  if (!fill) out_cnt[r] = count;
+  __syncwarp(gmask);
+  // transposed entry j: its column, value, lower bound in the direct row, and whether it goes out by itself
+  uint32_t c = 0, la = 0;
+  float b = 0.0f;
+  bool match = false, keep = false;
+  auto look = [&](uint64_t j) {
+    match = keep = false;
+    if (j >= jend) return;
+    const uint32_t pb = tvals[j];
+    b = pw[pb];
+    c = pb / k;
+    uint32_t lo = 0, hi = an;
+    while (lo < hi) {
+      const uint32_t mid = (lo + hi) >> 1;
+      if (s_c[mid] < c) lo = mid + 1;
+      else hi = mid;
+    }
+    la = lo;
+    match = lo < an && s_c[lo] == c;
+    keep = !match && __fmul_rn(mix, b) != 0.0f;
+  };
+  for (uint64_t jb = j0; jb < jend; jb += G) {
+    look(jb + gl);
+    if (match) s_b[la] = b;
+    if (keep) atomicAdd(&s_h[la], 1u);
+  }
+  __syncwarp(gmask);
+  uint32_t kept = 0, before = 0;  // direct entries kept, transpose-only ones, up to here
+  uint64_t o = fill ? out_ptr[r] : 0;
+  for (uint32_t ib = 0; ib <= an; ib += G) {
+    const uint32_t i = ib + gl;
+    float v = 0.0f;
+    if (i < an) {
+      const float a = s_a[i], tb = s_b[i];
+      v = __fadd_rn(__fadd_rn(__fmul_rn(mix, a), __fmul_rn(mix, tb)), __fmul_rn(__fmul_rn(prod, a), tb));
+    }
+    const uint32_t bits = (__ballot_sync(gmask, v != 0.0f) & gmask) >> shift;
+    uint32_t h = i <= an ? s_h[i] : 0;
+#pragma unroll
+    for (int d = 1; d < G; d <<= 1) {
+      const uint32_t u = __shfl_up_sync(gmask, h, d, G);
+      if (gl >= (uint32_t)d) h += u;
+    }
+    const uint32_t rank = kept + __popc(bits & below);
+    if (fill && v != 0.0f) {
+      out_idx[o + rank + before + h] = s_c[i];
+      out_w[o + rank + before + h] = v;
+    }
+    if (i <= an) s_h[i] = rank;
+    kept += __popc(bits);
+    before += __shfl_sync(gmask, h, G - 1, G);
+  }
+  if (!fill) {
+    if (gl == 0) out_cnt[r] = kept + before;
+    return;
+  }
+  __syncwarp(gmask);
+  const bool once = jend - j0 <= G;  // then the first look still holds
+  for (uint64_t jb = j0; jb < jend; jb += G) {
+    if (!once) look(jb + gl);
+    const uint32_t bits = (__ballot_sync(gmask, keep) & gmask) >> shift;
+    if (keep) {
+      const uint64_t at = o + s_h[la] + __popc(bits & below);
+      out_idx[at] = c;
+      out_w[at] = __fmul_rn(mix, b);
+    }
+    o += __popc(bits);
+  }
 }
 
 __global__ void empty_rows_kernel(const uint64_t* __restrict__ indptr, const float* __restrict__ data,
@@ -404,11 +472,17 @@ void smooth_knn(const float* dist, uint64_t n, uint64_t k, const GraphParams& gp
   UB_CUDA(cudaMemsetAsync(need.p, 0, sizeof(unsigned), s));
   const uint32_t stride = (uint32_t)k | 1u;
   const size_t smem = (size_t)BT * stride * sizeof(float);
-  const unsigned grid = grid_for(n, BT);
-  if (smem <= 48 * 1024) {
-    smooth_knn_kernel<true><<<grid, BT, smem, s>>>(dist, n, (uint32_t)k, gp, sigmas, rhos, need.p);
+  int dev = 0, sms = 0;
+  UB_CUDA(cudaGetDevice(&dev));
+  UB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  if (smem > 48 * 1024) {
+    smooth_knn_kernel<false, 1><<<grid_for(n, BT), BT, 0, s>>>(dist, n, (uint32_t)k, gp, sigmas, rhos, need.p);
+  } else if (n <= 128ull * (uint64_t)std::max(sms, 1)) {
+    smooth_knn_kernel<true, 16><<<grid_for(n, BT / 16), BT, smem / 8, s>>>(dist, n, (uint32_t)k, gp, sigmas, rhos, need.p);
+  } else if (n <= 256ull * (uint64_t)std::max(sms, 1)) {
+    smooth_knn_kernel<true, 4><<<grid_for(n, BT / 4), BT, smem / 2, s>>>(dist, n, (uint32_t)k, gp, sigmas, rhos, need.p);
   } else {
-    smooth_knn_kernel<false><<<grid, BT, 0, s>>>(dist, n, (uint32_t)k, gp, sigmas, rhos, need.p);
+    smooth_knn_kernel<true, 1><<<grid_for(n, BT), BT, smem, s>>>(dist, n, (uint32_t)k, gp, sigmas, rhos, need.p);
   }
   UB_LAUNCH_CHECK();
   segment_mean_kernel<<<n_seg, 32, 0, s>>>(dist, (uint32_t)k, seg ? seg->seg_off : nullptr, n, need.p, gmean.p);
@@ -457,8 +531,15 @@ void union_rows(const uint32_t* pcol, const float* pw, const uint32_t* cnt, uint
                 uint32_t* out_cnt, const uint64_t* out_ptr, uint32_t* out_idx, float* out_w,
                 bool fill, cudaStream_t s) {
   if (n == 0) return;
-  union_kernel<<<grid_for(n, BT), BT, 0, s>>>(pcol, pw, cnt, (uint32_t)k, tptr, tvals, n, gp.mix,
-                                              gp.prod_coeff, out_cnt, out_ptr, out_idx, out_w, fill);
+  auto launch = [&](auto kernel, unsigned lanes) {
+    const unsigned rows = BT / lanes;
+    kernel<<<grid_for(n, rows), BT, rows * 4 * (k + 1) * sizeof(uint32_t), s>>>(
+        pcol, pw, cnt, (uint32_t)k, tptr, tvals, n, gp.mix, gp.prod_coeff, out_cnt, out_ptr, out_idx, out_w, fill);
+  };
+  // Lanes per row (both launches and the sort before them, ms, 4 / 8 / 16 / 32 lanes): 2M x 15 4.4 / 3.3 /
+  // 3.0 / 3.2, 70k x 15 0.36 / 0.30 / 0.26 / 0.24, 30k x 30 0.42 / 0.29 / 0.22 / 0.20.
+  if (k <= 16) launch(union_kernel<16>, 16);
+  else launch(union_kernel<32>, 32);
   UB_LAUNCH_CHECK();
 }
 
