@@ -812,20 +812,24 @@ __global__ void kept_degree_kernel(const uint64_t* __restrict__ indptr, const fl
   deg[r] = c;
 }
 
-// Batched instances: max graph weight of each instance (optimizer.rs:90-94 per instance).
+// Batched instances: max graph weight of each instance (optimizer.rs:90-94 per instance).  gridDim.y
+// blocks share an instance and merge by its bits (the maximum is at least +0): 64 instances of 75k
+// edges took 357 us with a block each, 25 with 18.
 __global__ void segment_max_kernel(const uint64_t* __restrict__ indptr, const float* __restrict__ data,
-                                   const uint64_t* __restrict__ seg_off, float* __restrict__ out) {
+                                   const uint64_t* __restrict__ seg_off, int* __restrict__ out) {
   const uint32_t sgm = blockIdx.x;
   const uint64_t q0 = indptr[seg_off[sgm]], q1 = indptr[seg_off[sgm + 1]];
   float m = 0.0f;
-  for (uint64_t q = q0 + threadIdx.x; q < q1; q += blockDim.x) m = fmaxf(m, data[q]);
+  const uint64_t step = (uint64_t)gridDim.y * blockDim.x;
+#pragma unroll 4
+  for (uint64_t q = q0 + blockIdx.y * blockDim.x + threadIdx.x; q < q1; q += step) m = fmaxf(m, data[q]);
   __shared__ float s_m[32];
   for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xFFFFFFFFu, m, o));
   if ((threadIdx.x & 31) == 0) s_m[threadIdx.x >> 5] = m;
   __syncthreads();
   if (threadIdx.x == 0) {
     for (uint32_t w = 1; w < blockDim.x / 32; ++w) m = fmaxf(m, s_m[w]);
-    out[sgm] = m;
+    atomicMax(out + sgm, __float_as_int(m));
   }
 }
 
@@ -847,34 +851,42 @@ __global__ void ptr_degree_kernel(const uint64_t* __restrict__ kptr, uint64_t n,
 // over its length, in RATE_BITS bits), so that a warp's lanes draw similar numbers of firings
 // per epoch; batched instances sort instance-major first.
 constexpr int RATE_BITS = 8;
+// With rates, G = 16 lanes per row: the divisions of 16 edges at once, added up in their order (10k
+// points: 63 us with a thread per row, 18 with 16); without, G = 1.
+template <int G>
 __global__ void task_fill_kernel(const uint64_t* __restrict__ kptr, const uint32_t* __restrict__ deg,
                                  const uint64_t* __restrict__ tptr, uint64_t n, uint32_t chunk,
                                  const uint32_t* __restrict__ row_seg, int len_bits, int rate_bits,
                                  int block_shift, const double* __restrict__ keps, const uint32_t* __restrict__ order,
                                  uint32_t* __restrict__ trow, uint64_t* __restrict__ tstart,
                                  uint32_t* __restrict__ tkey) {
-  const uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const uint64_t r = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) / G;
   if (r >= n) return;
+  const uint32_t gl = threadIdx.x & (G - 1), gmask = ((1u << G) - 1u) << (threadIdx.x & 31 & ~(G - 1));
   const uint64_t src = order ? order[r] : r;  // the kept-edge CSR row of layout row r
   const uint32_t d = deg[r];
   const uint64_t t0 = tptr[r], nt = tptr[r + 1] - t0;
   for (uint64_t c = 0; c < nt; ++c) {
     const uint32_t len = (uint32_t)min((uint64_t)chunk, (uint64_t)d - c * chunk);
     const uint64_t st = kptr[src] + c * chunk;
-    trow[t0 + c] = (uint32_t)r | (nt > 1 ? 0x80000000u : 0u);   // high bit: partial row
-    tstart[t0 + c] = st;
     uint32_t rate = 0;
     if (rate_bits) {
       float sp = 0.0f;
-      for (uint32_t e = 0; e < len; ++e) {
-        const double x = keps[st + e];
-        sp += x > 1.0 ? (float)(1.0 / x) : (x > 0.0 ? 1.0f : 0.0f);
+      for (uint32_t e = 0; e < len; e += G) {
+        const double x = e + gl < len ? keps[st + e + gl] : 0.0;
+        const float p = x > 1.0 ? (float)(1.0 / x) : (x > 0.0 ? 1.0f : 0.0f);
+#pragma unroll
+        for (int i = 0; i < G; ++i) sp += __shfl_sync(gmask, p, i, G);  // past the end: + 0
       }
       const uint32_t top = (1u << rate_bits) - 1u;
       rate = top - min(top, (uint32_t)(sp / (float)max(len, 1u) * (float)(top + 1u)));
     }
     const uint32_t hi = block_shift >= 0 ? (uint32_t)(r >> block_shift) : (row_seg ? row_seg[r] : 0u);
-    tkey[t0 + c] = (((hi << len_bits) | (chunk - len)) << rate_bits) | rate;
+    if (gl == 0) {
+      trow[t0 + c] = (uint32_t)r | (nt > 1 ? 0x80000000u : 0u);   // high bit: partial row
+      tstart[t0 + c] = st;
+      tkey[t0 + c] = (((hi << len_bits) | (chunk - len)) << rate_bits) | rate;
+    }
   }
 }
 
@@ -904,28 +916,27 @@ __global__ void slice_meta_kernel(const uint32_t* __restrict__ perm, const uint3
   }
 }
 
+// The entries of the tasks: 8 lanes per task where a task's entries are contiguous, a lane per task where
+// they are interleaved, so that a warp's writes fill whole sectors in both (2M points, lane major: 708
+// us with a lane per task, 327 with 8).
 __global__ void slice_fill_kernel(const uint32_t* __restrict__ ktail, const double* __restrict__ keps,
                                   const uint32_t* __restrict__ perm, const uint64_t* __restrict__ tstart,
                                   const uint32_t* __restrict__ skey, uint64_t T, uint32_t chunk,
                                   int rate_bits, uint32_t len_mask, const uint64_t* __restrict__ wscan,
                                   const uint32_t* __restrict__ width, uint64_t n_slices, bool lane_major,
                                   const uint32_t* __restrict__ rank, uint2* __restrict__ entry) {
-  const uint64_t q = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, q = lane_major ? t >> 3 : t;
   if (q >= n_slices * 32) return;
   const uint64_t s = q >> 5;
-  const uint32_t lane = (uint32_t)(q & 31);
-  const uint64_t base = wscan[s] * 32;
-  const uint32_t wd = width[s];
-  uint32_t e = 0;
-  if (q < T) {
-    const uint64_t st = tstart[perm[q]];
-    const uint32_t len = chunk - ((skey[q] >> rate_bits) & len_mask);
-    for (; e < len; ++e)
-      entry[lane_major ? base + (uint64_t)lane * wd + e : base + (uint64_t)e * 32 + lane] =
-          make_uint2(rank ? rank[ktail[st + e]] : ktail[st + e], q_minus_1(keps[st + e]));
+  const uint32_t lane = (uint32_t)(q & 31), wd = width[s], step = lane_major ? 8 : 1;
+  const uint64_t base = wscan[s] * 32 + (lane_major ? (uint64_t)lane * wd : lane), stride = lane_major ? 1 : 32;
+  const uint64_t st = q < T ? tstart[perm[q]] : 0;
+  const uint32_t len = q < T ? chunk - ((skey[q] >> rate_bits) & len_mask) : 0u;
+  for (uint32_t e = lane_major ? (uint32_t)t & 7 : 0u; e < wd; e += step) {
+    uint2 v = make_uint2(0u, 0u);
+    if (e < len) v = make_uint2(rank ? rank[ktail[st + e]] : ktail[st + e], q_minus_1(keps[st + e]));
+    entry[base + e * stride] = v;
   }
-  for (; e < wd; ++e)
-    entry[lane_major ? base + (uint64_t)lane * wd + e : base + (uint64_t)e * 32 + lane] = make_uint2(0u, 0u);
 }
 
 __global__ void head_from_ptr_kernel(const uint64_t* __restrict__ kptr, uint64_t n, uint32_t* __restrict__ head) {
@@ -958,14 +969,18 @@ __device__ __forceinline__ double epochs_per_sample(float w, double max_w, doubl
   return n_samples > 0.0 ? n_ep / n_samples : -1.0;
 }
 
+// 8 lanes per row, their kept edges placed by rank, so that reads and writes fill sectors (2M points: 1117
+// us with a thread per row, 696 with 8 lanes).
 __global__ void export_edges_kernel(const uint64_t* __restrict__ indptr, const uint32_t* __restrict__ indices,
                                     const float* __restrict__ data, uint64_t n, float thr, double max_w,
                                     double n_ep, const float* __restrict__ seg_thr,
                                     const float* __restrict__ seg_maxw, const uint32_t* __restrict__ row_seg,
                                     const uint64_t* __restrict__ kept_ptr, uint32_t* __restrict__ head,
                                     uint32_t* __restrict__ tail, double* __restrict__ eps) {
-  const uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  constexpr uint32_t G = 8;
+  const uint64_t r = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) / G;
   if (r >= n) return;
+  const uint32_t gl = threadIdx.x & (G - 1), shift = threadIdx.x & 24, gmask = 0xFFu << shift;
   float t = thr;
   double mw = max_w;
   if (seg_thr) {
@@ -974,14 +989,20 @@ __global__ void export_edges_kernel(const uint64_t* __restrict__ indptr, const u
     mw = (double)seg_maxw[sg];
   }
   uint64_t o = kept_ptr[r];
-  for (uint64_t j = indptr[r]; j < indptr[r + 1]; ++j) {
-    const float w = data[j];
-    if (w >= t) {
-      if (head) head[o] = (uint32_t)r;
-      if (tail) tail[o] = indices[j];
-      if (eps) eps[o] = epochs_per_sample(w, mw, n_ep);
-      ++o;
+  const uint64_t jend = indptr[r + 1];
+  for (uint64_t jb = indptr[r]; jb < jend; jb += G) {
+    const uint64_t j = jb + gl;
+    const float w = j < jend ? data[j] : 0.0f;
+    const uint32_t k = tail && j < jend ? indices[j] : 0;
+    const bool keep = j < jend && w >= t;
+    const uint32_t bits = (__ballot_sync(gmask, keep) & gmask) >> shift;
+    if (keep) {
+      const uint64_t at = o + __popc(bits & ((1u << gl) - 1u));
+      if (head) head[at] = (uint32_t)r;
+      if (tail) tail[at] = k;
+      if (eps) eps[at] = epochs_per_sample(w, mw, n_ep);
     }
+    o += __popc(bits);
   }
 }
 
@@ -1149,7 +1170,9 @@ void kept_degree(const uint64_t* indptr, const float* data, uint64_t n, float th
 void segment_max(const uint64_t* indptr, const float* data, const uint64_t* seg_off, uint32_t n_seg,
                  float* out, cudaStream_t s) {
   if (n_seg == 0) return;
-  segment_max_kernel<<<n_seg, 256, 0, s>>>(indptr, data, seg_off, out);
+  UB_CUDA(cudaMemsetAsync(out, 0, n_seg * sizeof(float), s));
+  const unsigned parts = std::max(1u, std::min(64u, 1184u / n_seg));  // about 8 blocks per SM in all
+  segment_max_kernel<<<dim3(n_seg, parts), 256, 0, s>>>(indptr, data, seg_off, (int*)out);
   UB_LAUNCH_CHECK();
 }
 
@@ -1329,10 +1352,14 @@ void build_sgd_layout(const uint64_t* kept_ptr, const uint32_t* ktail, const dou
     block_bits = bits_for(n >> block_shift);
   }
   if (n) {
-    task_fill_kernel<<<grid_for(n, 256), 256, 0, s>>>(kept_ptr, deg.p, tptr.p, n, L.chunk,
-                                                      seg ? seg->row_seg : nullptr, len_bits, rate_bits, block_shift,
-                                                      keps, L.order.p, trow.p, tstart.p, tkey.p);
-    UB_LAUNCH_CHECK();
+    auto fill = [&](auto kernel, unsigned rows) {
+      kernel<<<grid_for(n, rows), 256, 0, s>>>(kept_ptr, deg.p, tptr.p, n, L.chunk, seg ? seg->row_seg : nullptr,
+                                               len_bits, rate_bits, block_shift, keps, L.order.p, trow.p, tstart.p,
+                                               tkey.p);
+      UB_LAUNCH_CHECK();
+    };
+    if (rate_bits) fill(task_fill_kernel<16>, 16);
+    else fill(task_fill_kernel<1>, 256);
   }
   if (T && torder == TaskOrder::Row) {
     iota_u32_kernel<<<grid_for(T, 256), 256, 0, s>>>(perm.p, T);
@@ -1361,7 +1388,7 @@ void build_sgd_layout(const uint64_t* kept_ptr, const uint32_t* ktail, const dou
   L.n_entries = wtot * 32;
   L.entry.alloc(L.n_entries, s);
   if (L.n_slices) {
-    slice_fill_kernel<<<grid_for(L.n_slices * 32, 256), 256, 0, s>>>(ktail, keps, perm.p, tstart.p, skey.p, T,
+    slice_fill_kernel<<<grid_for(L.n_slices * 32 * (L.lane_major ? 8 : 1), 256), 256, 0, s>>>(ktail, keps, perm.p, tstart.p, skey.p, T,
                                                                         L.chunk, rate_bits, len_mask, wscan.p,
                                                                         L.slice_width.p, L.n_slices,
                                                                         L.lane_major, rank.p, L.entry.p);
@@ -1383,7 +1410,7 @@ void export_edges(const uint64_t* indptr, const uint32_t* indices, const float* 
                   float thr, float max_w, uint64_t total_epochs, const uint64_t* kept_ptr,
                   uint32_t* head, uint32_t* tail, double* eps, cudaStream_t s, const SegmentPrune* sp) {
   if (n == 0) return;
-  export_edges_kernel<<<grid_for(n, 256), 256, 0, s>>>(
+  export_edges_kernel<<<grid_for(n, 32), 256, 0, s>>>(
       indptr, indices, data, n, thr, (double)max_w, (double)total_epochs, sp ? sp->seg_thr : nullptr,
       sp ? sp->seg_maxw : nullptr, sp ? sp->row_seg : nullptr, kept_ptr, head, tail, eps);
   UB_LAUNCH_CHECK();
