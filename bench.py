@@ -363,7 +363,7 @@ def run_reference(a):
 
 def run_batched(a):
     """Batched many-instance workload: one batched fit (one kernel launch per epoch over all
-    instances, graph-captured, autotuned) vs a per-instance loop of the plain fit.  With N
+    instances, autotuned) vs a per-instance loop of the plain fit.  With N
     ranks the instances are cut into N contiguous, edge-balanced shards (no data-path
     collective); value = all ranks' edge-updates / the slowest rank's time."""
     import torch
