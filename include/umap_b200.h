@@ -264,7 +264,8 @@ int umap_optimizer_tuning(const umap_optimizer* opt, uint32_t* chunk, uint32_t* 
  * task, tasks dealt by firings in blocks of 128), UMAP_LAYOUT_ROWS (a thread per task;
  * 5 to 7 components),
  * UMAP_LAYOUT_DRAM with _TWELVE_NEGATIVES (a lane per task, 12 row loads in flight; DRAM-bound layouts),
- * none of them: any number of components; UMAP_LAYOUT_EIGHT_NEGATIVES (no longer set),
+ * none of them: up to 4 components a lane per task (UMAP_LAYOUT_EIGHT_NEGATIVES: in its budget of 8 row
+ * loads in flight, in 1-D and 2-D; else 4), above that any number of components;
  * UMAP_LAYOUT_RENAMED (vertices renamed into a locality
  * order; DRAM-bound plain fits), UMAP_LAYOUT_GENERIC_RULE (the optimizer's MetricType is
  * Generic), and the order in which tasks are dealt to warps: UMAP_LAYOUT_RATE_ORDER (by

@@ -513,7 +513,7 @@ std::unique_ptr<umap_optimizer> optimizer_prepare_impl(std::unique_ptr<umap_mani
     compute_kept_edges(*o, K, true, true);
     log.mark("optimizer edge filtering + epochs_per_sample complete");
     const bool generic = o->metric_type == UMAP_METRIC_GENERIC;
-    build_sgd_layout(K.ptr.p, K.tail.p, K.eps.p, n, (uint32_t)dims, 0, generic, o->layout, s);
+    build_sgd_layout(K.ptr.p, K.tail.p, K.eps.p, n, (uint32_t)dims, 0, generic, o->initial_alpha, o->layout, s);
     log.mark("optimizer task layout complete");
   }
   if (log.on)
@@ -680,33 +680,40 @@ std::unique_ptr<umap_fitted> fit_impl(const umap_config& c, uint64_t n_samples, 
 }
 
 // ------------------------------------------------------------------ autotuning
-// Picks the SGD task length ("edges per thread") by timing two epochs of each candidate on a
-// scratch copy of the embedding.  Choices are cached per
-// problem size (vertices, edges in MiB units, dims) for the life of the process.
+// Picks the SGD task length ("edges per thread") and the lane kernel's block shape by timing two
+// epochs of each candidate on a scratch copy of the embedding.  Choices are cached per
+// problem size (vertices, edges in MiB units, dims) and kernel for the life of the process.
 struct TuneKey {
   uint64_t n, e_mib, dim;
+  EpochKernel kernel;
   bool operator<(const TuneKey& o) const {
-    return n != o.n ? n < o.n : e_mib != o.e_mib ? e_mib < o.e_mib : dim < o.dim;
+    return n != o.n ? n < o.n : e_mib != o.e_mib ? e_mib < o.e_mib : dim != o.dim ? dim < o.dim : kernel < o.kernel;
   }
 };
+struct Tuned {
+  uint32_t chunk, block_threads;
+};
 std::mutex& g_tune_mu = *new std::mutex;
-std::map<TuneKey, uint32_t>& g_tuned = *new std::map<TuneKey, uint32_t>;
+std::map<TuneKey, Tuned>& g_tuned = *new std::map<TuneKey, Tuned>;
 
 void tune_layout(umap_optimizer& o, const KeptEdges& K) {
   cudaStream_t s = o.s();
   const uint64_t n = o.manifold->n_vertices;
-  const TuneKey key{n, K.E >> 20, o.dim};
+  const TuneKey key{n, K.E >> 20, o.dim, pick_epoch_kernel(n, (uint32_t)o.dim, 0, false, true, false, o.initial_alpha)};
   Segments sgs{o.n_seg, o.seg_off.p, o.row_seg.p};
   const Segments* seg_ptr = o.n_seg ? &sgs : nullptr;
+  auto build = [&](uint32_t chunk, SgdLayout& L) {
+    build_sgd_layout(K.ptr.p, K.tail.p, K.eps.p, n, (uint32_t)o.dim, chunk, false, o.initial_alpha, L, s, seg_ptr);
+  };
   {
     std::lock_guard<std::mutex> lock(g_tune_mu);
     auto it = g_tuned.find(key);
     if (it != g_tuned.end()) {
-      build_sgd_layout(K.ptr.p, K.tail.p, K.eps.p, n, (uint32_t)o.dim, it->second, false, o.layout, s, seg_ptr);
+      build(it->second.chunk, o.layout);
+      o.layout.block_threads = it->second.block_threads;
       return;
     }
   }
-  const uint32_t chunks[] = {32, 64, 128, 256};
   const uint32_t mid = (uint32_t)std::max<uint64_t>(1, o.total_epochs / 2);
   DevBuf<float> scratch(2 * n * o.dim, s);
   d2d(scratch.p, o.emb2.p, n * o.dim, s);
@@ -716,30 +723,38 @@ void tune_layout(umap_optimizer& o, const KeptEdges& K) {
   UB_CUDA(cudaEventCreate(&e0));
   UB_CUDA(cudaEventCreate(&e1));
   float best = 1e30f;
-  uint32_t best_chunk = 0;
-  for (uint32_t ch : chunks) {
+  Tuned pick{0, 256};
+  for (uint32_t ch : {32u, 64u, 128u, 256u}) {
     SgdLayout L;
-    build_sgd_layout(K.ptr.p, K.tail.p, K.eps.p, n, (uint32_t)o.dim, ch, false, L, s, seg_ptr);
-    sgd_epoch(L, scratch.p, scratch.p + n * o.dim, p, mid, 0.5f, false, s);  // warm-up
-    UB_CUDA(cudaEventRecord(e0, s));
-    for (int r = 0; r < 2; ++r) sgd_epoch(L, scratch.p, scratch.p + n * o.dim, p, mid + r, 0.5f, r > 0, s);
-    UB_CUDA(cudaEventRecord(e1, s));
-    UB_CUDA(cudaEventSynchronize(e1));
-    float ms = 0;
-    UB_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-    if (ms < best) {
-      best = ms;
-      best_chunk = ch;
-      o.layout = std::move(L);
+    build(ch, L);
+    const uint32_t own = L.block_threads;
+    bool better = false;
+    for (uint32_t bt : {128u, 256u}) {
+      if (bt != own && L.kernel != EpochKernel::Lane) continue;
+      L.block_threads = bt;
+      sgd_epoch(L, scratch.p, scratch.p + n * o.dim, p, mid, 0.5f, false, s);  // warm-up
+      UB_CUDA(cudaEventRecord(e0, s));
+      for (int r = 0; r < 2; ++r) sgd_epoch(L, scratch.p, scratch.p + n * o.dim, p, mid + r, 0.5f, r > 0, s);
+      UB_CUDA(cudaEventRecord(e1, s));
+      UB_CUDA(cudaEventSynchronize(e1));
+      float ms = 0;
+      UB_CUDA(cudaEventElapsedTime(&ms, e0, e1));
+      if (ms < best) {
+        best = ms;
+        pick = {ch, bt};
+        better = true;
+      }
     }
+    if (better) o.layout = std::move(L);
     if (o.layout.max_degree <= ch) break;  // longer tasks would be the same whole rows
   }
+  o.layout.block_threads = pick.block_threads;
   (void)cudaEventDestroy(e0);
   (void)cudaEventDestroy(e1);
   if (getenv("UMAP_B200_LOG"))
-    fprintf(stderr, "[umap_b200] autotune: chunk=%u (%.3f ms / 2 epochs)\n", best_chunk, best);
+    fprintf(stderr, "[umap_b200] autotune: chunk=%u block=%u (%.3f ms / 2 epochs)\n", pick.chunk, pick.block_threads, best);
   std::lock_guard<std::mutex> lock(g_tune_mu);
-  g_tuned[key] = best_chunk;
+  g_tuned[key] = pick;
 }
 
 // ------------------------------------------------------------------ batched instances
@@ -841,11 +856,9 @@ std::unique_ptr<umap_optimizer> batch_new_impl(const umap_config& c, uint64_t n_
   {
     KeptEdges K;
     compute_kept_edges(*o, K, true, true);
-    static const bool no_tune = [] {
-      const char* e = getenv("UMAP_B200_AUTOTUNE");
-      return e && e[0] == '0';
-    }();
-    if (no_tune || total_epochs < 2) build_sgd_layout(K.ptr.p, K.tail.p, K.eps.p, N, (uint32_t)dims, 0, false, o->layout, s, &so);
+    const char* tune = getenv("UMAP_B200_AUTOTUNE");
+    if ((tune && tune[0] == '0') || total_epochs < 2) build_sgd_layout(K.ptr.p, K.tail.p, K.eps.p, N, (uint32_t)dims, 0, false, o->initial_alpha,
+                                                    o->layout, s, &so);
     else tune_layout(*o, K);
   }
   set_l2_window(*o, true);
@@ -1039,7 +1052,7 @@ void finish_loaded_optimizer(umap_optimizer& o, const DevBuf<uint32_t>& head, co
   DevBuf<uint64_t> ptr(n + 1, s);
   segment_starts(head.p, E, n, ptr.p, s);
   const bool generic = o.metric_type == UMAP_METRIC_GENERIC;
-  build_sgd_layout(ptr.p, tail.p, eps.p, n, (uint32_t)o.dim, 0, generic, o.layout, s);
+  build_sgd_layout(ptr.p, tail.p, eps.p, n, (uint32_t)o.dim, 0, generic, o.initial_alpha, o.layout, s);
   set_l2_window(o, true);
   UB_CUDA(cudaStreamSynchronize(s));
 }
@@ -2189,7 +2202,7 @@ int umap_optimizer_tuning(const umap_optimizer* opt, uint32_t* chunk, uint32_t* 
   API_BEGIN
   need(opt, "optimizer");
   if (chunk) *chunk = opt->layout.chunk;
-  if (block_threads) *block_threads = epoch_block_threads(opt->layout);
+  if (block_threads) *block_threads = opt->layout.block_threads;
   API_END
 }
 
@@ -2197,6 +2210,7 @@ int umap_optimizer_layout_flags(const umap_optimizer* opt, uint32_t* flags) {
   API_BEGIN
   need(opt, "optimizer"); need(flags, "flags");
   *flags = (opt->layout.lane_major ? UMAP_LAYOUT_LANE_MAJOR : 0u) |
+           (opt->layout.kernel == EpochKernel::Lane && opt->layout.short_epoch ? UMAP_LAYOUT_EIGHT_NEGATIVES : 0u) |
            (opt->layout.kernel == EpochKernel::Dram ? UMAP_LAYOUT_DRAM | UMAP_LAYOUT_TWELVE_NEGATIVES : 0u) |
            (opt->layout.kernel == EpochKernel::Pool ? UMAP_LAYOUT_POOLED : 0u) |
            (opt->layout.kernel == EpochKernel::Rows ? UMAP_LAYOUT_ROWS : 0u) |

@@ -44,6 +44,13 @@ constexpr uint32_t PAD_ROW = 0xFFFFFFFFu;
 // 295.1, 12 / 3: 295.2, 12 / 2: 313.4, 16 / 2: 316.0, 24 / 2: 317.7; 40M points, 24 epochs:
 // 8 / 4: 590.4, 12 / 3: 562.6, 16 / 2: 564.9).
 constexpr int NB_DRAM = 12, MINB_DRAM = 3;
+// The lane kernel (sgd_epoch_kernel2) comes in two register budgets.  Large graphs (many waves of
+// warps): 4 negative rows fetched together and 5 resident 256-thread blocks per SM.  Graphs that
+// fill about two waves or fewer are bound by the chain of dependent loads of their busiest lanes: 8
+// negative rows fetched together and 4 blocks per SM.  (2M points, 500 epochs, SGD ms: 4 / 5 314.0, 8 / 4
+// 317.6, 6 / 4 330.9, 4 / 4 343.5.)
+constexpr int NB_WIDE = 4, MINB_WIDE = 5;
+constexpr int NB_SHORT = 8, MINB_SHORT = 4;
 // The pooled kernel: 8 negative rows fetched together, 8 blocks of 128 threads per SM (64
 // registers).  2M points, us per epoch: 8 / 8: 482, 6 / 8: 480, 6 / 9: 481, 4 / 10: 516, 4 / 8: 511;
 // 300k points: 92, 98, 98, 106, 106.
@@ -288,6 +295,7 @@ template <int DIM, bool GEN, int NEG_BATCH>
 __device__ __forceinline__ void fired_edge(float (&cur)[DIM], uint32_t r, uint32_t k, uint32_t nneg,
                                            float* snap, const SgdParams& p, float alpha, uint64_t idx,
                                            uint32_t epoch, uint32_t seg_lo, uint32_t seg_n) {
+  const float a = p.a, b = p.b;
   float* oth = snap + (uint64_t)k * DIM;
   float o[DIM];
   load_row<DIM>(o, oth);
@@ -323,20 +331,31 @@ __device__ __forceinline__ void fired_edge(float (&cur)[DIM], uint32_t r, uint32
   };
   fetch(0);
   // attractive step (:284-306)
+  float ds = 0.0f;
+#pragma unroll
+  for (int d = 0; d < DIM; ++d) { const float df = cur[d] - o[d]; ds += df * df; }
   float g[DIM];
   if constexpr (GEN) {
     // head += clip(c * grad) alpha; tail += clip(c * rev_grad) alpha with rev_grad = -grad
-    float ds = 0.0f, den;
+    float den;
+    const float gc = metric_coeff(ds, a, p.two_b, p.two_b, -1.0f, &den);
 #pragma unroll
-    for (int d = 0; d < DIM; ++d) { const float df = cur[d] - o[d]; ds += df * df; }
-    const float gc = metric_coeff(ds, p.a, p.two_b, p.two_b, -1.0f, &den);
-#pragma unroll
-    for (int d = 0; d < DIM; ++d) g[d] = clip4(gc * __fdividef(cur[d] - o[d], den)) * alpha;
+    for (int d = 0; d < DIM; ++d) {
+      g[d] = clip4(gc * __fdividef(cur[d] - o[d], den)) * alpha;
+      cur[d] += g[d];
+    }
   } else {
-    attract<DIM>(cur, o, g, p, alpha);
-  }
+    float gc = 0.0f;
+    if (ds > 0.0f) {
+      const float pb = __powf(ds, b);
+      gc = __fdividef(p.neg_attr * pb, ds * (a * pb * ds + 1.0f));
+    }
 #pragma unroll
-  for (int d = 0; d < DIM; ++d) cur[d] += g[d];
+    for (int d = 0; d < DIM; ++d) {
+      g[d] = clip4(gc * (cur[d] - o[d])) * alpha;
+      cur[d] += g[d];
+    }
+  }
   sub_row<DIM>(oth, g);
   // negative samples (:313-341)
   for (uint32_t q0 = 0; q0 < nneg; q0 += NEG_BATCH) {
@@ -345,16 +364,131 @@ __device__ __forceinline__ void fired_edge(float (&cur)[DIM], uint32_t r, uint32
     for (int q = 0; q < NEG_BATCH; ++q) {
       if (q0 + q >= nneg) break;
       if (kk[q] == r) continue;
-      if constexpr (GEN) {
-        float dsn = 0.0f, den;
+      if constexpr (DIM == 2 && !GEN) {
+        // the same operations as the generic-DIM code below, two columns per instruction
+        const uint64_t c2 = pk2(cur[0], cur[1]);
+        const uint64_t df2 = sub2(c2, pk2(ob[q][0], ob[q][1]));
+        float df0, df1;
+        up2(df2, df0, df1);
+        const float dsn = df0 * df0 + df1 * df1;
+        float gr = 0.0f;
+        if (dsn > 0.0f) {
+          const float pb = __powf(dsn, b);
+          gr = __fdividef(p.pos_rep, (0.001f + dsn) * (a * pb * dsn + 1.0f));
+        }
+        if (gr > 0.0f) {
+          float t0, t1;
+          up2(mul2(pk2(gr, gr), df2), t0, t1);
+          up2(fma2(pk2(clip4(t0), clip4(t1)), pk2(alpha, alpha), c2), cur[0], cur[1]);
+        }
+        continue;
+      }
+      float dsn = 0.0f;
 #pragma unroll
-        for (int d = 0; d < DIM; ++d) { const float df = cur[d] - ob[q][d]; dsn += df * df; }
-        const float gr = metric_coeff(dsn, p.a, p.two_b, p.pos_rep, 0.0f, &den);
+      for (int d = 0; d < DIM; ++d) { const float df = cur[d] - ob[q][d]; dsn += df * df; }
+      if constexpr (GEN) {
+        float den;
+        const float gr = metric_coeff(dsn, a, p.two_b, p.pos_rep, 0.0f, &den);
 #pragma unroll
         for (int d = 0; d < DIM; ++d) cur[d] += clip4(gr * __fdividef(cur[d] - ob[q][d], den)) * alpha;
       } else {
-        repel<DIM>(cur, ob[q], true, p, alpha);
+        float gr = 0.0f;
+        if (dsn > 0.0f) {
+          const float pb = __powf(dsn, b);
+          gr = __fdividef(p.pos_rep, (0.001f + dsn) * (a * pb * dsn + 1.0f));
+        }
+        if (gr > 0.0f) {
+#pragma unroll
+          for (int d = 0; d < DIM; ++d) cur[d] += clip4(gr * (cur[d] - ob[q][d])) * alpha;
+        }
       }
+    }
+  }
+}
+
+// A lane per task with independent progress: each lane walks its own task through a small register
+// window of entries (refilled on demand, 4 loads in flight), so a warp runs as long as its busiest
+// task rather than its busiest lane of every batch.  Its order of updates is the one that layouts
+// at small learning rates keep (see pick_epoch_kernel).
+template <int DIM, bool GEN, int NEG_BATCH, int MINB, bool LM, bool SEG>
+__global__ void __launch_bounds__(256, MINB) sgd_epoch_kernel2(
+    const uint64_t* __restrict__ slice_base, const uint32_t* __restrict__ slice_width,
+    const uint32_t* __restrict__ split_mask, const uint32_t* __restrict__ rowid,
+    const uint2* __restrict__ entry, uint64_t n_slices, float* __restrict__ live, float* snap,
+    SgdParams p, uint32_t epoch, float alpha) {
+  constexpr int W = 4;
+  const uint64_t slice = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const uint32_t lane = threadIdx.x & 31;
+  if (slice >= n_slices) return;
+  const uint32_t r = rowid[slice * 32 + lane];
+  const bool active = r != PAD_ROW;
+  const uint32_t width = active ? slice_width[slice] : 0u;
+  const uint64_t base = slice_base[slice];
+  const bool split = (split_mask[slice] >> lane) & 1u;
+  uint32_t seg_lo = 0, seg_n = p.n_vertices;
+  if constexpr (SEG) {
+    if (active) {
+      const uint32_t sg = p.row_seg[r];
+      seg_lo = (uint32_t)p.seg_off[sg];
+      seg_n = (uint32_t)(p.seg_off[sg + 1] - p.seg_off[sg]);
+    }
+  }
+  float cur[DIM], start[DIM];
+  float* hrow = live + (uint64_t)(active ? r : 0) * DIM;
+  if (active) load_row<DIM>(cur, hrow);
+  else
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) cur[d] = 0.0f;
+#pragma unroll
+  for (int d = 0; d < DIM; ++d) start[d] = cur[d];
+  const uint32_t n = epoch;
+  static_assert(W % 4 == 0, "windows are whole 4-entry sectors");
+  // this lane's entries: contiguous (lane major) or every 32nd (interleaved)
+  const uint2* lent = LM ? entry + base + (uint64_t)lane * width : entry + base + lane;
+  uint2 win[W];
+  uint32_t mask = 0, ew = 0, ebase = 0;
+  for (;;) {
+    while (mask == 0 && ew < width) {
+      ebase = ew;
+      if (LM) {
+        // width is a multiple of W (slice_meta_kernel): the window lies inside the lane's entries
+#pragma unroll
+        for (int j = 0; j < W; j += 2) {
+          const uint4 v = __ldg(reinterpret_cast<const uint4*>(lent + ew + j));
+          win[j] = make_uint2(v.x, v.y);
+          win[j + 1] = make_uint2(v.z, v.w);
+        }
+      } else {
+#pragma unroll
+        for (int j = 0; j < W; ++j) {
+          const uint32_t e = ew + j;
+          win[j] = e < width ? __ldg(lent + (uint64_t)e * 32) : make_uint2(0u, 0u);
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < W; ++j)
+        if (fires_at(n, win[j].y)) mask |= 1u << j;
+      ew += W;
+    }
+    if (!__any_sync(0xFFFFFFFFu, mask != 0)) break;
+    if (mask) {
+      const int j = __ffs(mask) - 1;
+      mask &= mask - 1;
+      uint2 en = win[0];
+#pragma unroll
+      for (int t = 1; t < W; ++t)
+        if (t == j) en = win[t];
+      const uint32_t nneg = negatives_at(n, en.y, p.neg_rate);
+      const uint64_t idx = LM ? base + (uint64_t)lane * width + ebase + j : base + (uint64_t)(ebase + j) * 32 + lane;
+      fired_edge<DIM, GEN, NEG_BATCH>(cur, r, en.x, nneg, snap, p, alpha, idx, epoch, seg_lo, seg_n);
+    }
+  }
+  if (active) {
+    if (split) {
+#pragma unroll
+      for (int d = 0; d < DIM; ++d) atomicAdd(hrow + d, cur[d] - start[d]);
+    } else {
+      store_row<DIM>(hrow, cur);
     }
   }
 }
@@ -639,7 +773,7 @@ __global__ void __launch_bounds__(256) sgd_epoch_anydim(
     const uint64_t* __restrict__ slice_base, const uint32_t* __restrict__ slice_width,
     const uint32_t* __restrict__ split_mask, const uint32_t* __restrict__ rowid,
     const uint2* __restrict__ entry, uint64_t n_slices, float* __restrict__ live, float* snap,
-    SgdParams p, uint32_t epoch, float alpha) {
+    SgdParams p, uint32_t epoch, float alpha, bool lane_major) {
   const uint64_t slice = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint32_t lane = threadIdx.x & 31;
   if (slice >= n_slices) return;
@@ -664,7 +798,7 @@ __global__ void __launch_bounds__(256) sgd_epoch_anydim(
     else cur[d] += v;
   };
   for (uint32_t e = 0; e < width; ++e) {
-    const uint64_t idx = base + (uint64_t)lane * width + e;
+    const uint64_t idx = lane_major ? base + (uint64_t)lane * width + e : base + (uint64_t)e * 32 + lane;
     const uint2 en = __ldcs(entry + idx);
     if (!fires_at(n, en.y)) continue;
     float* oth = snap + (uint64_t)en.x * dim;
@@ -1230,36 +1364,82 @@ uint32_t pick_chunk_generic(uint64_t n_edges) {
   return std::max<uint32_t>(64, pick_chunk(n_edges));
 }
 
-// Graphs of at most two waves of a lane per task at 40 warps per SM: their tasks are ordered by firing
-// rate too (pick_task_order).
-bool small_graph(uint64_t n_slices) {
+int sm_count() {
   int dev = 0, sms = 0;
   UB_CUDA(cudaGetDevice(&dev));
   UB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  return n_slices <= 2ull * (uint64_t)std::max(sms, 1) * 40;
+  return std::max(sms, 1);
+}
+
+// Graphs of at most two waves of a lane per task at 40 warps per SM: their tasks are ordered by firing
+// rate too (pick_task_order), and the lane kernel takes its 8-negatives budget in 1-D and 2-D.
+// UMAP_B200_SGD_SHORT=0 / 1 forces it, and with it the lane kernel (1-D to 4-D).
+bool small_graph(uint64_t n_slices) {
+  if (const char* e = getenv("UMAP_B200_SGD_SHORT")) {
+    if (e[0] == '0') return false;
+    if (e[0] == '1') return true;
+  }
+  return n_slices <= 2ull * (uint64_t)sm_count() * 40;
 }
 
 // The epoch kernel of a layout.
-//  * Rows / AnyDim: rows of 5 to 7 and of more columns.  Forces of 8-D layouts and up are so small
-//    that the order of the updates, which every faster kernel changes, shows in the result: 30k
-//    points in 8-D differ between the two kernels by 2e-4 of their size, between two runs of AnyDim
-//    by 4e-5 (6-D: 2e-4 and 6e-5, 5-D: 2.4e-4 and 9e-5).
 //  * Dram: renamed 1-D and 2-D layouts whose snapshot (4 * dim bytes per vertex) is above 80 MB, so
 //    that with the edge stream it does not stay in the 126 MB L2.  The random rows then cost DRAM
 //    bursts, and the interleaved order's whole 256-byte rows per warp use them better than a task's
 //    contiguous entries (2-D rolls, 30 epochs, Dram interleaved against Pool lane major, ms: 5M points
 //    34.7 / 28.2, 8M 55.1 / 44.6, 12M 94.6 / 98.7, 16M 149.6 / 156.9, 20M 207.2 / 221.6).
-//  * Pool: everything else.
-// UMAP_B200_SGD_KERNEL=pool / dram forces one that can run the layout.
-EpochKernel pick_epoch_kernel(uint64_t n, uint32_t dim, bool renamed, bool segmented, bool generic) {
-  if (dim > 4) return dim <= 7 && !generic ? EpochKernel::Rows : EpochKernel::AnyDim;
-  const bool can_dram = dim <= 2 && !generic && !segmented;
-  if (const char* e = getenv("UMAP_B200_SGD_KERNEL")) {
-    if (!strcmp(e, "dram") && can_dram) return EpochKernel::Dram;
-    if (!strcmp(e, "pool")) return EpochKernel::Pool;
+//  * Pool (1-D to 4-D) and Rows (5-D to 7-D, Euclidean rule): layouts at learning rates from which on
+//    the epochs' races decide the result.  Lane and AnyDim: the others.
+//    The kernels draw the same samples and make the same moves, but which updates of an epoch see
+//    which differs between them, the same way in every epoch.  At small rates the races of one kernel
+//    nearly average out and this difference does not: the median relative distance between runs of
+//    Pool and of Lane, over that between two runs of Lane, is, at rate 0.002, 4.3 at 200k, 4.6 at 1M
+//    and 2.6 at 2M points; at 0.006, 2.2 to 2.9 at 500, in 3-D 3.9 at 2,000; at 0.01, 1.7 at 300 to 1,500,
+//    1.5 at 10k, 1.7 at 70k, in batches 1.6 to 2.3, in 3-D 2.0 at 10k; in 2-D at 0.05, 1.0 to 1.4; in 3-D at
+//    0.1, 1.1 to 1.3, at 0.3, 1.0; Rows against AnyDim in 5-D: 4.6 at 500 and 2.8 at 100k at 0.01, 1.1 to 2.4
+//    at 0.03, 1.0 at 0.3.  The lines are the rates from which on runs of the two kernels are within four
+//    times the distance between two runs of one as often as those runs themselves: RACING_RATE for plain 1-D
+//    and 2-D Euclidean layouts of at least POOL_MIN_SLICES slices per SM (7,500 points of 25 neighbours
+//    hold it, 3,000 of 15 do not, 22% of the pairs against 3%), RACING_RATE_WIDE for the rest.
+//    Renamed layouts take Pool at every rate: their locality order alone moves two runs as far apart as
+//    the kernels (5M points: 7.2e-3 either way).
+//    Time, Lane / Pool, ms per fit: 10k points 7.3 / 4.4, 70k 9.1 / 6.9, 1M 35.4 / 28.2, 64 instances
+//    23.6 / 16.7; AnyDim / Rows, 20k points in 5-D 50 / 11.
+// UMAP_B200_SGD_KERNEL=lane / pool / dram / rows / any forces one that can run the layout.
+constexpr float RACING_RATE = 0.01f, RACING_RATE_WIDE = 0.03f;
+constexpr double POOL_MIN_SLICES = 2.5;
+constexpr uint64_t LANE_MAJOR_MAX = 4000000;
+EpochKernel pick_epoch_kernel(uint64_t n, uint32_t dim, uint64_t n_slices, bool renamed, bool segmented, bool generic,
+                              float alpha) {
+  const char* e = getenv("UMAP_B200_SGD_KERNEL");
+  const auto forced = [&](const char* name) { return e && !strcmp(e, name); };
+  if (dim > 4) {
+    if (dim > 7 || generic || forced("any")) return EpochKernel::AnyDim;
+    return forced("rows") || alpha >= RACING_RATE_WIDE ? EpochKernel::Rows : EpochKernel::AnyDim;
   }
+  const bool can_dram = dim <= 2 && !generic && !segmented;
+  if (forced("dram") && can_dram) return EpochKernel::Dram;
+  if (forced("pool")) return EpochKernel::Pool;
+  if (forced("lane") || getenv("UMAP_B200_SGD_SHORT")) return EpochKernel::Lane;
   if (can_dram && renamed && n * dim * 4 > 80000000ull) return EpochKernel::Dram;
-  return EpochKernel::Pool;
+  if (renamed) return EpochKernel::Pool;
+  if (!segmented && n > LANE_MAJOR_MAX) return EpochKernel::Lane;  // interleaved entries
+  const bool early = can_dram && (double)n_slices >= POOL_MIN_SLICES * sm_count();
+  return alpha >= (early ? RACING_RATE : RACING_RATE_WIDE) ? EpochKernel::Pool : EpochKernel::Lane;
+}
+
+// Entry order of the layout: lane major, or interleaved for Dram and, above 4M vertices of a plain fit,
+// for the kernels that take either (their random rows go to DRAM there, whose bursts whole 256-byte rows
+// per warp use better than a lane's 32-byte windows).  UMAP_B200_SGD_LANE_MAJOR=0 / 1 forces those.
+bool lane_major_entries(uint64_t n, bool segmented, EpochKernel kernel) {
+  if ((kernel == EpochKernel::Lane && !segmented) || kernel == EpochKernel::AnyDim) {
+    if (const char* e = getenv("UMAP_B200_SGD_LANE_MAJOR")) {
+      if (e[0] == '0') return false;
+      if (e[0] == '1') return true;
+    }
+    return segmented || n <= LANE_MAJOR_MAX;
+  }
+  return kernel != EpochKernel::Dram;
 }
 
 // Whether a plain fit's layout renames its vertices into a locality order (order.cu): from the
@@ -1275,7 +1455,7 @@ bool pick_relabel(uint64_t n, bool segmented) {
     if (e[0] == '0') return false;
     if (e[0] == '1') return true;
   }
-  return n > 4000000ull;
+  return n > LANE_MAJOR_MAX;
 }
 
 // Order in which the tasks are dealt to warps (32 consecutive tasks per warp):
@@ -1308,7 +1488,7 @@ TaskOrder pick_task_order(bool renamed, bool short_graph, bool segmented) {
 }
 
 void build_sgd_layout(const uint64_t* kept_ptr, const uint32_t* ktail, const double* keps, uint64_t n, uint32_t dim,
-                      uint32_t chunk, bool generic, SgdLayout& L, cudaStream_t s, const Segments* seg) {
+                      uint32_t chunk, bool generic, float alpha, SgdLayout& L, cudaStream_t s, const Segments* seg) {
   L.n_vertices = n;
   DevBuf<uint32_t> rank;
   L.order.reset();
@@ -1345,9 +1525,11 @@ void build_sgd_layout(const uint64_t* kept_ptr, const uint32_t* ktail, const dou
   if ((uint64_t)n_seg << len_bits >= (1ull << 32)) throw Error(UNSUPPORTED, "too many instances for the task sort key");
   const int seg_bits = n_seg ? bits_for(n_seg) : 0;
   const bool renamed = L.order.p != nullptr;
-  L.kernel = pick_epoch_kernel(n, dim, renamed, seg != nullptr, generic);
-  L.lane_major = L.kernel != EpochKernel::Dram;
-  TaskOrder torder = pick_task_order(renamed, small_graph((T + 31) / 32), seg != nullptr);
+  L.kernel = pick_epoch_kernel(n, dim, (T + 31) / 32, renamed, seg != nullptr, generic, alpha);
+  L.block_threads = L.kernel == EpochKernel::Pool ? POOL_BT : 256;
+  L.short_epoch = small_graph((T + 31) / 32);
+  L.lane_major = lane_major_entries(n, seg != nullptr, L.kernel);
+  TaskOrder torder = pick_task_order(renamed, L.short_epoch, seg != nullptr);
   if (torder == TaskOrder::LengthRate && len_bits + seg_bits + RATE_BITS > 32) torder = TaskOrder::Length;
   L.task_order = torder;
   const int rate_bits = torder == TaskOrder::LengthRate ? RATE_BITS : 0;
@@ -1443,8 +1625,6 @@ void normalize_init(float* emb, uint64_t n, uint32_t dim, cudaStream_t s, const 
   UB_LAUNCH_CHECK();
 }
 
-uint32_t epoch_block_threads(const SgdLayout& L) { return L.kernel == EpochKernel::Pool ? POOL_BT : 256; }
-
 // Launches an epoch kernel; `overlap` makes it a programmatic dependent of the launch before it on
 // the stream (only kernels that wait for that launch with grid_wait take it).
 template <class... P, class... A>
@@ -1483,6 +1663,10 @@ void sgd_epoch(const SgdLayout& L, float* live, float* snap, const SgdParams& p,
     launch_epoch(k, g, POOL_BT, overlap, s, UB_SGD_ARGS, g > 8000u);
   };
   const bool gen = p.generic_metric;
+  auto variants = [&](auto dims) {  // dims(generic rule, batch)
+    if (gen) p.row_seg ? dims(std::true_type{}, std::true_type{}) : dims(std::true_type{}, std::false_type{});
+    else p.row_seg ? dims(std::false_type{}, std::true_type{}) : dims(std::false_type{}, std::false_type{});
+  };
   switch (L.kernel) {
     case EpochKernel::Pool: {
       auto dims = [&](auto gen, auto seg) {
@@ -1491,8 +1675,23 @@ void sgd_epoch(const SgdLayout& L, float* live, float* snap, const SgdParams& p,
         else if (p.dim == 3) pooled(sgd_epoch_pool<3, gen.value, seg.value>);
         else pooled(sgd_epoch_pool<4, gen.value, seg.value>);
       };
-      if (gen) p.row_seg ? dims(std::true_type{}, std::true_type{}) : dims(std::true_type{}, std::false_type{});
-      else p.row_seg ? dims(std::false_type{}, std::true_type{}) : dims(std::false_type{}, std::false_type{});
+      variants(dims);
+      break;
+    }
+    case EpochKernel::Lane: {
+      const unsigned bt = L.block_threads;
+      auto lanes = [&](auto k) { launch_epoch(k, blocks(tasks, bt), bt, false, s, UB_SGD_ARGS); };
+      auto dims = [&](auto gen, auto seg, auto lm) {
+        constexpr bool G = gen.value, S = seg.value, LM = lm.value;
+        const bool eight = L.short_epoch && !G;
+        if (p.dim == 1) lanes(eight ? sgd_epoch_kernel2<1, false, NB_SHORT, MINB_SHORT, LM, S> : sgd_epoch_kernel2<1, G, NB_WIDE, MINB_WIDE, LM, S>);
+        else if (p.dim == 2) lanes(eight ? sgd_epoch_kernel2<2, false, NB_SHORT, MINB_SHORT, LM, S> : sgd_epoch_kernel2<2, G, NB_WIDE, MINB_WIDE, LM, S>);
+        else if (p.dim == 3) lanes(sgd_epoch_kernel2<3, G, NB_WIDE, MINB_WIDE, LM, S>);
+        else lanes(sgd_epoch_kernel2<4, G, NB_WIDE, MINB_WIDE, LM, S>);
+      };
+      if (L.lane_major) variants([&](auto gen, auto seg) { dims(gen, seg, std::true_type{}); });
+      else if (gen) dims(std::true_type{}, std::false_type{}, std::false_type{});
+      else dims(std::false_type{}, std::false_type{}, std::false_type{});
       break;
     }
     case EpochKernel::Rows:
@@ -1503,7 +1702,8 @@ void sgd_epoch(const SgdLayout& L, float* live, float* snap, const SgdParams& p,
       launch_epoch(p.dim == 1 ? sgd_epoch_dram<1> : sgd_epoch_dram<2>, blocks(tasks, BT), BT, false, s, UB_SGD_ARGS);
       break;
     case EpochKernel::AnyDim:
-      launch_epoch(gen ? sgd_epoch_anydim<true> : sgd_epoch_anydim<false>, blocks(tasks, BT), BT, false, s, UB_SGD_ARGS);
+      launch_epoch(gen ? sgd_epoch_anydim<true> : sgd_epoch_anydim<false>, blocks(tasks, BT), BT, false, s, UB_SGD_ARGS,
+                   L.lane_major);
       break;
   }
 #undef UB_SGD_ARGS

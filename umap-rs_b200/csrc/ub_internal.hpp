@@ -182,12 +182,14 @@ constexpr uint64_t MAX_EPOCHS = 1ull << 21;
 enum class TaskOrder { Length, LengthRate, RowBlock, Row };
 
 // Which kernel runs the layout's epochs (sgd.cu, pick_epoch_kernel).
-enum class EpochKernel { Pool, Rows, AnyDim, Dram };
+enum class EpochKernel { Lane, Pool, Rows, AnyDim, Dram };
 
 struct SgdLayout {
   uint64_t n_vertices = 0, n_edges = 0, n_entries = 0, n_slices = 0, n_tasks = 0;
   uint32_t max_degree = 0, chunk = 0;
-  EpochKernel kernel = EpochKernel::Pool;
+  EpochKernel kernel = EpochKernel::Lane;
+  uint32_t block_threads = 256;  // threads per block of the epoch kernel (multiple of 32)
+  bool short_epoch = false;      // a graph of at most ~2 waves of warps (sgd.cu, small_graph)
   bool lane_major = true;        // entry order: lane major (true) or interleaved by lane
   TaskOrder task_order = TaskOrder::Length;
   uint64_t split_tasks = 0;
@@ -251,12 +253,13 @@ void export_state(const double* eps, uint64_t E, uint64_t neg_rate, uint64_t cur
 // the one for the generic-metric rule, whose rows must stay whole tasks (see sgd.cu).
 uint32_t pick_chunk(uint64_t n_edges);
 uint32_t pick_chunk_generic(uint64_t n_edges);
-// `rename`: a plain fit's layout may rename its vertices into a locality order (DRAM-bound
-// sizes); the generic-metric rule passes false.
+EpochKernel pick_epoch_kernel(uint64_t n, uint32_t dim, uint64_t n_slices, bool renamed, bool segmented, bool generic,
+                              float alpha);
+// `alpha`: the initial learning rate, which decides between the epoch kernels.  A plain fit's layout may
+// rename its vertices into a locality order (DRAM-bound sizes), but not under the generic-metric rule.
 void build_sgd_layout(const uint64_t* kept_ptr, const uint32_t* tail, const double* eps, uint64_t n, uint32_t dim,
-                      uint32_t chunk, bool generic, SgdLayout& L, cudaStream_t s, const Segments* seg = nullptr);
-// Threads per block of the layout's epoch kernel.
-uint32_t epoch_block_threads(const SgdLayout& L);
+                      uint32_t chunk, bool generic, float alpha, SgdLayout& L, cudaStream_t s,
+                      const Segments* seg = nullptr);
 void kept_degree(const uint64_t* indptr, const float* data, uint64_t n, float thr,
                  uint32_t* deg, cudaStream_t s, const SegmentPrune* sp = nullptr);
 // K6 normalise init into [0, 10] per dimension (optimizer.rs:181-230), in place.

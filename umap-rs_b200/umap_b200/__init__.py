@@ -652,8 +652,8 @@ class Optimizer(_Handle):
         return Optimizer(None, _handle=out.value)
 
     def layout(self) -> dict:
-        """How the SGD layout is laid out: lane-major entries, the 8-negatives register
-        budget, vertices renamed into a locality order, the order tasks are dealt to warps
+        """How the SGD layout is laid out: lane-major entries, the lane kernel's 8-negatives
+        register budget, vertices renamed into a locality order, the order tasks are dealt to warps
         ("length", "length+rate", "row blocks" or "rows"); and the epoch kernel it selects."""
         f = C.c_uint32()
         _check(_lib.load().umap_optimizer_layout_flags(self._get(), C.byref(f)))
