@@ -23,6 +23,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cfloat>
 #include <cstdint>
 #include <cstdlib>
 #include <cstring>
@@ -232,8 +233,10 @@ __device__ __forceinline__ float metric_coeff(float ds, float a, float two_b, fl
 // The Euclidean rule's step of a head row (optimize_layout_euclidean.rs:284-306, :319-339) with
 // the shortest chain from the row to its update, which is what a task's firings wait for: the
 // squared distance carries the smallest normal number along (a subnormal one would cost scaling
-// instructions around each approximate log2 / exp2 / reciprocal; the move at such a distance is
-// below 1e-16 either way), ds^b = 2^(b log2 ds), and the denominators are one fused step behind it.
+// instructions around each approximate log2 / exp2 / reciprocal), ds^b = 2^(b log2 ds), and the
+// denominators are one fused step behind it.  Like the rule, an attraction at distance 0 or NaN has
+// coefficient 0 and a repulsion moves only where its coefficient is above 0 (it is 0 at an infinite
+// distance): a row with a NaN or infinite coordinate leaves those that draw it alone.
 __device__ __forceinline__ float ftz_log2(float x) { float r; asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
 __device__ __forceinline__ float ftz_exp2(float x) { float r; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
 __device__ __forceinline__ float ftz_rcp(float x) { float r; asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
@@ -246,16 +249,16 @@ __device__ __forceinline__ float clip4(float v) {
 }
 template <int DIM>
 __device__ __forceinline__ float square_ftz(const float (&df)[DIM]) {
-  float ds = 1.17549435e-38f;
+  float ds = FLT_MIN;
 #pragma unroll
   for (int d = 0; d < DIM; ++d) ds = fmaf(df[d], df[d], ds);
   return ds;
 }
-// Attraction coefficient -2ab ds^b / (ds (a ds^b ds + 1)) as num * inv.
-__device__ __forceinline__ void attract_terms(float ds, const SgdParams& p, float& num, float& inv) {
+// Attraction coefficient -2ab ds^b / (ds (a ds^b ds + 1)), of square_ftz's distance.
+__device__ __forceinline__ float attract_coeff(float ds, const SgdParams& p) {
   const float pb = ftz_exp2(p.b * ftz_log2(ds));
-  num = p.neg_attr * pb;
-  inv = ftz_rcp(fmaf(p.a * ds * ds, pb, ds));
+  const float c = (p.neg_attr * pb) * ftz_rcp(fmaf(p.a * ds * ds, pb, ds));
+  return ds > FLT_MIN ? c : 0.0f;
 }
 // 1 / ((0.001 + ds)(a ds^b ds + 1)), the repulsion coefficient over 2 gamma b.
 __device__ __forceinline__ float repel_inv(float ds, const SgdParams& p) {
@@ -266,22 +269,21 @@ __device__ __forceinline__ float repel_inv(float ds, const SgdParams& p) {
 template <int DIM>
 __device__ __forceinline__ void attract(float (&cur)[DIM], const float (&o)[DIM], float (&g)[DIM], const SgdParams& p,
                                         float alpha) {
-  float df[DIM], num, inv;
-#pragma unroll
-  for (int d = 0; d < DIM; ++d) df[d] = cur[d] - o[d];
-  attract_terms(square_ftz<DIM>(df), p, num, inv);
-#pragma unroll
-  for (int d = 0; d < DIM; ++d) g[d] = clip4((num * df[d]) * inv) * alpha;
-}
-// Repulsive move from row o, where `apply`; a NaN distance (a NaN row) moves nothing.
-template <int DIM>
-__device__ __forceinline__ void repel(float (&cur)[DIM], const float (&o)[DIM], bool apply, const SgdParams& p,
-                                      float alpha) {
   float df[DIM];
 #pragma unroll
   for (int d = 0; d < DIM; ++d) df[d] = cur[d] - o[d];
-  const float ds = square_ftz<DIM>(df), inv = repel_inv(ds, p);
-  if (apply && ds > 0.0f) {
+  const float c = attract_coeff(square_ftz<DIM>(df), p);
+#pragma unroll
+  for (int d = 0; d < DIM; ++d) g[d] = clip4(c * df[d]) * alpha;
+}
+// Repulsive move from row o.
+template <int DIM>
+__device__ __forceinline__ void repel(float (&cur)[DIM], const float (&o)[DIM], const SgdParams& p, float alpha) {
+  float df[DIM];
+#pragma unroll
+  for (int d = 0; d < DIM; ++d) df[d] = cur[d] - o[d];
+  const float inv = repel_inv(square_ftz<DIM>(df), p);
+  if (p.pos_rep * inv > 0.0f) {
 #pragma unroll
     for (int d = 0; d < DIM; ++d) cur[d] = fmaf(clip4((p.pos_rep * df[d]) * inv), alpha, cur[d]);
   }
@@ -741,14 +743,14 @@ __global__ void __launch_bounds__(POOL_BT, MINB_POOL) sgd_epoch_pool(
           sub_row<DIM>(oth, g);
 #pragma unroll
           for (int q = 0; q < NB_POOL; ++q)
-            if ((ok >> q) & 1u) repel<DIM>(cur, ob[q], true, p, alpha);
+            if ((ok >> q) & 1u) repel<DIM>(cur, ob[q], p, alpha);
           const NegRng rng(p.seed, at, epoch);
           for (uint32_t q = NB_POOL; q < drawn; ++q) {  // more negatives than fetched together
             const uint64_t rnd = rng.pair(q >> 1);
             const uint32_t k = seg_lo + __umulhi((q & 1) ? (uint32_t)(rnd >> 32) : (uint32_t)rnd, seg_n);
             if (k == row) continue;
             load_row_l2<DIM>(o, snap + (uint64_t)k * DIM);
-            repel<DIM>(cur, o, true, p, alpha);
+            repel<DIM>(cur, o, p, alpha);
           }
         }
       }
@@ -792,7 +794,7 @@ __global__ void __launch_bounds__(256) sgd_epoch_anydim(
   float* cur = live + (uint64_t)r * dim;
   const uint32_t n = epoch;
   const uint64_t seed = p.seed;
-  const float a = p.a;
+  const float a = p.a, b = p.b;
   auto add = [&](uint32_t d, float v) {
     if (split) atomicAdd(cur + d, v);
     else cur[d] += v;
@@ -807,10 +809,9 @@ __global__ void __launch_bounds__(256) sgd_epoch_anydim(
     float gc = 0.0f, den = 1.0f;
     if constexpr (GEN) {
       gc = metric_coeff(ds, a, p.two_b, p.two_b, -1.0f, &den);
-    } else {
-      float num, inv;
-      attract_terms(ds + 1.17549435e-38f, p, num, inv);
-      gc = num * inv;
+    } else if (ds > 0.0f) {
+      const float pb = __powf(ds, b);
+      gc = __fdividef(p.neg_attr * pb, ds * (a * pb * ds + 1.0f));
     }
     for (uint32_t d = 0; d < dim; ++d) {
       const float cd = cur[d], od = oth[d];
@@ -834,7 +835,11 @@ __global__ void __launch_bounds__(256) sgd_epoch_anydim(
         const float gr = metric_coeff(dsn, a, p.two_b, p.pos_rep, 0.0f, &dn);
         for (uint32_t d = 0; d < dim; ++d) add(d, clip4(gr * __fdividef(cur[d] - ob[d], dn)) * alpha);
       } else {
-        const float gr = p.pos_rep * repel_inv(dsn + 1.17549435e-38f, p);
+        float gr = 0.0f;
+        if (dsn > 0.0f) {
+          const float pb = __powf(dsn, b);
+          gr = __fdividef(p.pos_rep, (0.001f + dsn) * (a * pb * dsn + 1.0f));
+        }
         if (gr > 0.0f)
           for (uint32_t d = 0; d < dim; ++d) add(d, clip4(gr * (cur[d] - ob[d])) * alpha);
       }
@@ -911,12 +916,7 @@ __global__ void __launch_bounds__(256) sgd_epoch_rows(
       fetch(0);
       // attractive step (optimize_layout_euclidean.rs:284-306)
       {
-        float num, inv;
-#pragma unroll
-        for (int d = 0; d < DIM; ++d) df[d] = cur[d] - o[d];
-        attract_terms(square_ftz<DIM>(df), p, num, inv);
-#pragma unroll
-        for (int d = 0; d < DIM; ++d) g[d] = clip4((num * df[d]) * inv) * alpha;
+        attract<DIM>(cur, o, g, p, alpha);
         move(g);
         sub_row<DIM>(oth, g);
       }
@@ -929,8 +929,8 @@ __global__ void __launch_bounds__(256) sgd_epoch_rows(
           if (split) load_row_l2<DIM>(cur, hrow);
 #pragma unroll
           for (int d = 0; d < DIM; ++d) df[d] = cur[d] - x[q][d];
-          const float ds = square_ftz<DIM>(df), inv = repel_inv(ds, p);
-          if (!(ds > 0.0f)) continue;  // a NaN distance (a NaN row) moves nothing
+          const float inv = repel_inv(square_ftz<DIM>(df), p);
+          if (!(p.pos_rep * inv > 0.0f)) continue;
 #pragma unroll
           for (int d = 0; d < DIM; ++d) g[d] = clip4((p.pos_rep * df[d]) * inv) * alpha;
           move(g);
