@@ -1098,13 +1098,12 @@ void exact_rows(const float* X, int64_t n, int d, int k, const uint32_t* rows, u
 //    keeps HC = 32: 4 splits up to k = 64, else 8, for at most 8 of the k on average (the points within
 //    the error margin of the k-th come on top).  A row whose list overflows fails its certificate and
 //    is recomputed exactly.
-//  * Fewer than LONG_LIST_MIN points and k > KNN_MAX_K: the exact path, as before (1,500 x 40, k = 100:
-//    2.3 ms; 2,500 points through the candidate pass 0.5 ms): callers of sets this small read
-//    rows_recomputed = n.
+//  * Fewer than LONG_LIST_MIN points and k > KNN_MAX_K: the exact path, which the interface states
+//    (rows_recomputed = n; 1,500 x 40, k = 100: 2.3 ms, 2,500 points through the candidate pass 0.5 ms).
 constexpr uint64_t LONG_LIST_MIN = 2048;
-int pick_splits(uint64_t k, int64_t q_blocks, int64_t tiles, int sms) {
+int pick_splits(uint64_t n, uint64_t k, int64_t q_blocks, int64_t tiles, int sms) {
   if (k > (uint64_t)KNN_MAX_K) {
-    if (tiles * DBN < (int64_t)LONG_LIST_MIN) return 0;
+    if (n < LONG_LIST_MIN) return 0;
     return k <= 64 ? 4 : 8;
   }
   const int counts[] = {1, 2, 3, 4, 6, 8};
@@ -1173,7 +1172,7 @@ KnnStats knn_bruteforce(const float* X, uint64_t n, uint64_t d, uint64_t k, uint
   int cur = 0, sms = 148;
   UB_CUDA(cudaGetDevice(&cur));
   UB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, cur));
-  const int S = pick_splits(k, q_blocks, tiles, sms);
+  const int S = pick_splits(n, k, q_blocks, tiles, sms);
   st.splits = (uint32_t)S;
 
   DevBuf<double> sums(d, s);
