@@ -15,3 +15,16 @@ def test_long_lists_of_small_sets_are_exact(ub, oracle, n, exact):
     oi, od = oracle.knn_bruteforce(X, 100)
     assert np.array_equal(gi, oi) and np.array_equal(gd, od)
     assert rec == n if exact else rec < n // 20
+
+
+@pytest.mark.parametrize("n,classes,k", [(4097, 8, 60), (8000, 16, 100), (16383, 16, 128), (20480, 16, 100)])
+def test_alternating_classes(ub, oracle, n, classes, k):
+    """Row i in class i % classes, a period that a deal of the caller's order would send to one list: only the few
+    rows whose error margin overflows a list are recomputed."""
+    g = np.random.Generator(np.random.PCG64(classes))
+    X = (g.standard_normal((n, 16)) + 20.0 * g.standard_normal((classes, 16))[np.arange(n) % classes]).astype(np.float32)
+    gi, gd, rec = ub.knn_bruteforce(X, k, return_stats=True)
+    r1 = min(n, 500)
+    oi, od = oracle.knn_bruteforce(X, k, rows=(0, r1))
+    assert np.array_equal(gi[:r1], oi) and np.array_equal(gd[:r1], od)
+    assert rec < n // 20
