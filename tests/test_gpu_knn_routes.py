@@ -28,3 +28,15 @@ def test_alternating_classes(ub, oracle, n, classes, k):
     oi, od = oracle.knn_bruteforce(X, k, rows=(0, r1))
     assert np.array_equal(gi[:r1], oi) and np.array_equal(gd[:r1], od)
     assert rec < n // 20
+
+
+@pytest.mark.parametrize("n,d,k,rows", [(3000, 12, 10, 128), (2500, 20, 25, 1024), (2600, 8, 100, 640), (20001, 6, 15, 4096),
+                                        (17000, 5, 50, 3072), (2304, 9, 15, 2176), (2049, 9, 15, 2176)])
+def test_rows_in_several_passes(ub, monkeypatch, n, d, k, rows):
+    """The candidates of some rows at a time (a last pass of few rows, one row, or padding only; with and without a
+    locality order): the same result as all at once."""
+    X = _data(n, d, seed=n, kind="clusters")
+    want = ub.knn_bruteforce(X, k)
+    monkeypatch.setenv("UMAP_B200_KNN_ROWS", str(rows))
+    got = ub.knn_bruteforce(X, k)
+    assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])

@@ -45,6 +45,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
+#include <cstdlib>
 #include <cstring>
 #include <mutex>
 
@@ -365,11 +366,12 @@ __device__ __noinline__ ListState thin_list(const float* ld, uint32_t occ0, uint
 }
 
 // Persistent: CTA b takes the work items b, b + gridDim.x, ... of q_blocks x n_splits (query block,
-// split); split s scans the tiles s, s + n_splits, ...
+// split); split s scans the tiles s, s + n_splits, ...  The query blocks are the q_blocks from q_first on, and the
+// candidate arrays hold their rows only, in scan order.
 template <int RL>
 __global__ void __launch_bounds__(KNN_THREADS, 1) knn_candidates_kernel(
     const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tdb, const float* __restrict__ nb,
-    int64_t n, int n_kchunks, int64_t tiles_total, int64_t q_blocks, int n_splits, int k, int d,
+    int64_t n, int n_kchunks, int64_t tiles_total, int64_t q_first, int64_t q_blocks, int n_splits, int k, int d,
     const unsigned* __restrict__ rmax_bits, float gamma, float scale, const uint32_t* __restrict__ perm,
     uint32_t* __restrict__ list_idx, uint32_t* __restrict__ cand_idx, float* __restrict__ cand_d,
     float* __restrict__ tau_out, unsigned* __restrict__ err) {
@@ -393,10 +395,10 @@ __global__ void __launch_bounds__(KNN_THREADS, 1) knn_candidates_kernel(
   struct Item {
     int64_t m0, w0;
     int split, T, wn, S;
-    __device__ __forceinline__ Item(int64_t w, int64_t q_blocks, int n_splits, int64_t tiles) {
+    __device__ __forceinline__ Item(int64_t w, int64_t q_first, int64_t q_blocks, int n_splits, int64_t tiles) {
       split = (int)(w / q_blocks);
       S = n_splits;
-      m0 = (w - (int64_t)split * q_blocks) * QM;
+      m0 = (q_first + w - (int64_t)split * q_blocks) * QM;
       T = (int)((tiles - split + n_splits - 1) / n_splits);
       int64_t own = m0 / DBN / n_splits - WIN / 2;
       own = own < 0 ? 0 : own;
@@ -443,7 +445,7 @@ __global__ void __launch_bounds__(KNN_THREADS, 1) knn_candidates_kernel(
       int64_t g = 0, tt = 0, n_issued = 0;
       bool ok = true;
       for (int64_t w = blockIdx.x; w < items && ok; w += gridDim.x) {
-        const Item it(w, q_blocks, n_splits, tiles_total);
+        const Item it(w, q_first, q_blocks, n_splits, tiles_total);
         for (int t = 0; t < it.T && ok; ++t, ++tt) {
           const int64_t tile = it.tile(t);
           for (int c = 0; c < n_kchunks; ++c, ++g) {
@@ -491,7 +493,7 @@ __global__ void __launch_bounds__(KNN_THREADS, 1) knn_candidates_kernel(
       int64_t g = 0, tt = 0;
       bool ok = true;
       for (int64_t w = blockIdx.x; w < items && ok; w += gridDim.x) {
-        const int T = Item(w, q_blocks, n_splits, tiles_total).T;
+        const int T = Item(w, q_first, q_blocks, n_splits, tiles_total).T;
         for (int t = 0; t < T && ok; ++t, ++tt) {
           const int buf = (int)(tt & 1);
           if (tt >= 2 && !mbar_wait(smem_u32(&tempty[buf]), (uint32_t)(((tt >> 1) - 1) & 1))) {
@@ -554,7 +556,7 @@ __global__ void __launch_bounds__(KNN_THREADS, 1) knn_candidates_kernel(
     int slot4 = 0;
     bool ok = true;
     for (int64_t w = blockIdx.x; w < items && ok; w += gridDim.x, slot4 = (slot4 + 1) & 3) {
-      const Item it(w, q_blocks, n_splits, tiles_total);
+      const Item it(w, q_first, q_blocks, n_splits, tiles_total);
       const int64_t row = it.m0 + trow;
       const bool live = row < n;
       const float nq = live ? nb[row] : 0.0f;
@@ -717,9 +719,8 @@ __global__ void __launch_bounds__(KNN_THREADS, 1) knn_candidates_kernel(
       if (!ok) break;
       thin();
       mine[lane] = INFINITY;
-      if (live) {  // outputs by original row index, candidates as original indices
-        const int64_t orow = perm ? (int64_t)perm[row] : row;
-        const int64_t base = (orow * n_splits + it.split) * NCAND + half * HC;
+      if (live) {  // candidates as original indices
+        const int64_t at = (row - q_first * QM) * n_splits + it.split, base = at * NCAND + half * HC;
         for (int s = 0; s < HC; ++s) {
           const bool low = occ0 != 0, any = low || occ1 != 0;
           const int slot = low ? __ffs(occ0) - 1 : __ffs(occ1) + 31;
@@ -729,7 +730,7 @@ __global__ void __launch_bounds__(KNN_THREADS, 1) knn_candidates_kernel(
           cand_idx[base + s] = (perm && any) ? perm[c] : c;
           cand_d[base + s] = any ? ld[slot * QM] : INFINITY;
         }
-        tau_out[(orow * n_splits + it.split) * 2 + half] = tau;
+        tau_out[at * 2 + half] = tau;
       }
     }
   }
@@ -803,7 +804,8 @@ __device__ __forceinline__ float ref_distance_warp(const float* __restrict__ X, 
 constexpr int RERANK_BT = 128;
 template <int E>  // candidates per lane = splits * NCAND / 32
 __global__ void __launch_bounds__(RERANK_BT) knn_rerank_kernel(
-    const float* __restrict__ X, int64_t n, int d, int dp, int k, const uint32_t* __restrict__ cand_idx,
+    const float* __restrict__ X, int64_t n, int64_t first, int64_t count, int d, int dp, int k,
+    const uint32_t* __restrict__ cand_idx,
     const float* __restrict__ cand_d, const float* __restrict__ tau_in, const float* __restrict__ rn,
     const unsigned* __restrict__ rmax_bits, float gamma, float scale, const uint32_t* __restrict__ order,
     uint32_t* __restrict__ out_idx, float* __restrict__ out_d, uint32_t* __restrict__ fail_rows,
@@ -818,18 +820,18 @@ __global__ void __launch_bounds__(RERANK_BT) knn_rerank_kernel(
   const float R = __uint_as_float(*rmax_bits);
   const int64_t w0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t w = w0; w < n; w += nw) {
+  for (int64_t w = w0; w < count; w += nw) {
     // rows in locality order when there is one: neighbouring warps share candidate rows in L2
-    const int64_t row = order ? (int64_t)order[w] : w;
+    const int64_t row = order ? (int64_t)order[first + w] : first + w;
     const float xr = rn[row];
     uint32_t ci[E];
     float ca[E], lo = INFINITY, hi = -INFINITY;
     int have = 0;
 #pragma unroll
     for (int e = 0; e < E; ++e) {
-      ci[e] = cand_idx[row * (S * NCAND) + e * 32 + lane];
+      ci[e] = cand_idx[w * (S * NCAND) + e * 32 + lane];
       const bool valid = ci[e] < (uint64_t)n;
-      ca[e] = valid ? cand_d[row * (S * NCAND) + e * 32 + lane] : INFINITY;
+      ca[e] = valid ? cand_d[w * (S * NCAND) + e * 32 + lane] : INFINITY;
       if (valid) {
         lo = fminf(lo, ca[e]);
         hi = fmaxf(hi, ca[e]);
@@ -904,7 +906,7 @@ __global__ void __launch_bounds__(RERANK_BT) knn_rerank_kernel(
     }
     if (lane == 0) {
       float tau = INFINITY;
-      for (int s = 0; s < 2 * S; ++s) tau = fminf(tau, tau_in[row * 2 * S + s]);  // (split, half)
+      for (int s = 0; s < 2 * S; ++s) tau = fminf(tau, tau_in[w * 2 * S + s]);  // (split, half)
       if (tau < INFINITY) {
         const float lb = distance_lower_bound(tau, xr, R, gamma, scale, d, dp);
         if (last == ~0ull || !(__uint_as_float((uint32_t)(last >> 32)) < lb))
@@ -1142,12 +1144,20 @@ int pick_splits(uint64_t n, uint64_t k, int64_t q_blocks, int64_t tiles, int sms
   return best;
 }
 
+// Rows whose candidates a call holds at once (a multiple of QM): 512 bytes a row and split, so that the
+// scratch of the longest lists (8 splits) stays below 8 GB at any n.  UMAP_B200_KNN_ROWS sets it.
+int64_t candidate_rows(int splits) {
+  int64_t rows = ((int64_t)8 << 30) / (splits * (int64_t)(NCAND * 8 + 8));
+  if (const char* e = getenv("UMAP_B200_KNN_ROWS")) rows = atoll(e);
+  return std::max<int64_t>(1, rows / QM) * QM;
+}
+
 template <int E>
-void launch_rerank(const float* X, int64_t n, int d, int dp, int k, const uint32_t* ci, const float* cd, const float* tau,
-                   const float* rn, const unsigned* rmax, float gamma, float scale, const uint32_t* order,
-                   uint32_t* oi, float* od, uint32_t* fr, unsigned* fc, cudaStream_t s) {
-  knn_rerank_kernel<E><<<blocks_for(n * 32, RERANK_BT), RERANK_BT, 0, s>>>(X, n, d, dp, k, ci, cd, tau, rn, rmax, gamma, scale,
-                                                               order, oi, od, fr, fc);
+void launch_rerank(const float* X, int64_t n, int64_t first, int64_t count, int d, int dp, int k, const uint32_t* ci,
+                   const float* cd, const float* tau, const float* rn, const unsigned* rmax, float gamma, float scale,
+                   const uint32_t* order, uint32_t* oi, float* od, uint32_t* fr, unsigned* fc, cudaStream_t s) {
+  knn_rerank_kernel<E><<<blocks_for(count * 32, RERANK_BT), RERANK_BT, 0, s>>>(
+      X, n, first, count, d, dp, k, ci, cd, tau, rn, rmax, gamma, scale, order, oi, od, fr, fc);
   UB_LAUNCH_CHECK();
 }
 
@@ -1276,45 +1286,52 @@ KnnStats knn_bruteforce(const float* X, uint64_t n, uint64_t d, uint64_t k, uint
                                             n >= KNN_REORDER_MIN ? nullptr : rn.p, flags.p + 1);
   UB_LAUNCH_CHECK();
 
-  const unsigned grid = (unsigned)std::min<int64_t>(q_blocks * S, sms);
+  const int64_t q_step = std::min<int64_t>(q_blocks, candidate_rows(S) / QM);
+  const uint64_t held = std::min<uint64_t>(n, (uint64_t)q_step * QM);
   const float gamma = (float)(dp + 8) * 9.5367432e-7f;  // (Dp + 8) 2^-20
-  DevBuf<uint32_t> cidx(n * S * NCAND, s), lidx((uint64_t)grid * 2 * CAP * QM, s);
-  DevBuf<float> cdist(n * S * NCAND, s), tau(n * S * 2, s);
+  DevBuf<uint32_t> cidx(held * S * NCAND, s), fail_rows(n, s);
+  DevBuf<uint32_t> lidx((uint64_t)std::min<int64_t>(q_step * S, sms) * 2 * CAP * QM, s);
+  DevBuf<float> cdist(held * S * NCAND, s), tau(held * S * 2, s);
   const CUtensorMap tq = bf16_tile_map(xh.p, n_pad, dp, dp, QM, true);
   const CUtensorMap tdb = bf16_tile_map(xh.p, n_pad, dp, dp, DBN, true);
-  cudaEvent_t ev[2];
-  UB_CUDA(cudaEventCreate(&ev[0]));
-  UB_CUDA(cudaEventCreate(&ev[1]));
-  UB_CUDA(cudaEventRecord(ev[0], s));
   auto candidates = k <= 16                    ? knn_candidates_kernel<8>
                     : k <= (uint64_t)KNN_MAX_K ? knn_candidates_kernel<16>
                                                : knn_candidates_kernel<0>;
-  candidates<<<grid, KNN_THREADS, KNN_SMEM, s>>>(tq, tdb, nb.p, (int64_t)n, (int)(dp / KC), tiles, q_blocks, S,
-                                                            (int)k, di, flags.p + 1, gamma, scale, perm.p, lidx.p, cidx.p, cdist.p, tau.p, flags.p + 2);
-  UB_LAUNCH_CHECK();
-  UB_CUDA(cudaEventRecord(ev[1], s));
-  unsigned kerr = 0;
-  UB_CUDA(cudaMemcpyAsync(&kerr, flags.p + 2, 4, cudaMemcpyDeviceToHost, s));
-  UB_CUDA(cudaStreamSynchronize(s));
-  (void)cudaEventElapsedTime(&st.candidate_ms, ev[0], ev[1]);
+  const int ki = (int)k, dpi = (int)dp;
+  cudaEvent_t ev[2];
+  UB_CUDA(cudaEventCreate(&ev[0]));
+  UB_CUDA(cudaEventCreate(&ev[1]));
+  for (int64_t q0 = 0; q0 < q_blocks; q0 += q_step) {
+    const int64_t first = q0 * QM, qn = std::min(q_step, q_blocks - q0), count = std::min((int64_t)n - first, qn * QM);
+    if (count <= 0) break;  // a last block of padding rows
+    UB_CUDA(cudaEventRecord(ev[0], s));
+    candidates<<<(unsigned)std::min<int64_t>(qn * S, sms), KNN_THREADS, KNN_SMEM, s>>>(
+        tq, tdb, nb.p, (int64_t)n, (int)(dp / KC), tiles, q0, qn, S, ki, di, flags.p + 1, gamma, scale, perm.p, lidx.p,
+        cidx.p, cdist.p, tau.p, flags.p + 2);
+    UB_LAUNCH_CHECK();
+    UB_CUDA(cudaEventRecord(ev[1], s));
+    unsigned kerr = 0;
+    UB_CUDA(cudaMemcpyAsync(&kerr, flags.p + 2, 4, cudaMemcpyDeviceToHost, s));
+    UB_CUDA(cudaStreamSynchronize(s));
+    float ms = 0.0f;
+    (void)cudaEventElapsedTime(&ms, ev[0], ev[1]);
+    st.candidate_ms += ms;
+    if (kerr) throw Error(CUDA, "kNN candidate pass: a pipeline wait timed out");
+    auto rerank = [&](auto launch) {
+      launch(X, (int64_t)n, first, count, di, dpi, ki, cidx.p, cdist.p, tau.p, rn.p, flags.p + 1, gamma, scale, perm.p,
+             out_idx, out_dist, fail_rows.p, flags.p + 3, s);
+    };
+    switch (S) {
+      case 1: rerank(launch_rerank<2>); break;
+      case 2: rerank(launch_rerank<4>); break;
+      case 3: rerank(launch_rerank<6>); break;
+      case 4: rerank(launch_rerank<8>); break;
+      case 6: rerank(launch_rerank<12>); break;
+      default: rerank(launch_rerank<16>); break;
+    }
+  }
   (void)cudaEventDestroy(ev[0]);
   (void)cudaEventDestroy(ev[1]);
-  if (kerr) throw Error(CUDA, "kNN candidate pass: a pipeline wait timed out");
-
-  DevBuf<uint32_t> fail_rows(n, s);
-  const int ki = (int)k, dpi = (int)dp;
-  auto rerank = [&](auto launch) {
-    launch(X, (int64_t)n, di, dpi, ki, cidx.p, cdist.p, tau.p, rn.p, flags.p + 1, gamma, scale, perm.p, out_idx, out_dist,
-           fail_rows.p, flags.p + 3, s);
-  };
-  switch (S) {
-    case 1: rerank(launch_rerank<2>); break;
-    case 2: rerank(launch_rerank<4>); break;
-    case 3: rerank(launch_rerank<6>); break;
-    case 4: rerank(launch_rerank<8>); break;
-    case 6: rerank(launch_rerank<12>); break;
-    default: rerank(launch_rerank<16>); break;
-  }
   unsigned n_fail = 0;
   UB_CUDA(cudaMemcpyAsync(&n_fail, flags.p + 3, 4, cudaMemcpyDeviceToHost, s));
   UB_CUDA(cudaStreamSynchronize(s));
