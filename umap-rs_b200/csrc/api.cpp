@@ -682,7 +682,8 @@ std::unique_ptr<umap_fitted> fit_impl(const umap_config& c, uint64_t n_samples, 
 // ------------------------------------------------------------------ autotuning
 // Picks the SGD task length ("edges per thread") and the lane kernel's block shape by timing two
 // epochs of each candidate on a scratch copy of the embedding.  Choices are cached per
-// problem size (vertices, edges in MiB units, dims) and kernel for the life of the process.
+// problem size (vertices, edges in MiB units, dims) and kernel for the life of the process; one
+// whose search ended at a task length that holds every row stands for batches with rows as short.
 struct TuneKey {
   uint64_t n, e_mib, dim;
   EpochKernel kernel;
@@ -691,7 +692,7 @@ struct TuneKey {
   }
 };
 struct Tuned {
-  uint32_t chunk, block_threads;
+  uint32_t chunk, block_threads, max_degree;
 };
 std::mutex& g_tune_mu = *new std::mutex;
 std::map<TuneKey, Tuned>& g_tuned = *new std::map<TuneKey, Tuned>;
@@ -705,14 +706,17 @@ void tune_layout(umap_optimizer& o, const KeptEdges& K) {
   auto build = [&](uint32_t chunk, SgdLayout& L) {
     build_sgd_layout(K.ptr.p, K.tail.p, K.eps.p, n, (uint32_t)o.dim, chunk, false, o.initial_alpha, L, s, seg_ptr);
   };
+  Tuned pick{0, 256, UINT32_MAX};
   {
     std::lock_guard<std::mutex> lock(g_tune_mu);
     auto it = g_tuned.find(key);
-    if (it != g_tuned.end()) {
-      build(it->second.chunk, o.layout);
-      o.layout.block_threads = it->second.block_threads;
-      return;
-    }
+    if (it != g_tuned.end()) pick = it->second;
+  }
+  if (pick.chunk) {
+    build(pick.chunk, o.layout);
+    o.layout.block_threads = pick.block_threads;
+    if (o.layout.max_degree <= pick.max_degree) return;
+    pick = Tuned{0, 256, UINT32_MAX};
   }
   const uint32_t mid = (uint32_t)std::max<uint64_t>(1, o.total_epochs / 2);
   DevBuf<float> scratch(2 * n * o.dim, s);
@@ -723,7 +727,6 @@ void tune_layout(umap_optimizer& o, const KeptEdges& K) {
   UB_CUDA(cudaEventCreate(&e0));
   UB_CUDA(cudaEventCreate(&e1));
   float best = 1e30f;
-  Tuned pick{0, 256};
   for (uint32_t ch : {32u, 64u, 128u, 256u}) {
     SgdLayout L;
     build(ch, L);
@@ -741,12 +744,16 @@ void tune_layout(umap_optimizer& o, const KeptEdges& K) {
       UB_CUDA(cudaEventElapsedTime(&ms, e0, e1));
       if (ms < best) {
         best = ms;
-        pick = {ch, bt};
+        pick.chunk = ch;
+        pick.block_threads = bt;
         better = true;
       }
     }
     if (better) o.layout = std::move(L);
-    if (o.layout.max_degree <= ch) break;  // longer tasks would be the same whole rows
+    if (o.layout.max_degree <= ch) {  // longer tasks would be the same whole rows
+      pick.max_degree = ch;
+      break;
+    }
   }
   o.layout.block_threads = pick.block_threads;
   (void)cudaEventDestroy(e0);
