@@ -292,8 +292,9 @@ __device__ __forceinline__ void repel(float (&cur)[DIM], const float (&o)[DIM], 
 // One fired edge (optimize_layout_euclidean.rs:278-343, or with GEN the generic-metric rule
 // of optimize_layout_generic.rs:57-121): attractive step on (head, tail), then `nneg`
 // negative samples, all reading the snapshot buffer.  The tail row and a batch of negative
-// rows are fetched together before the (sequential) updates of `cur`.
-template <int DIM, bool GEN, int NEG_BATCH>
+// rows are fetched together before the (sequential) updates of `cur`.  FUSED takes the Euclidean rule's moves from
+// attract / repel above; without it every operation stands by itself.
+template <int DIM, bool GEN, int NEG_BATCH, bool FUSED>
 __device__ __forceinline__ void fired_edge(float (&cur)[DIM], uint32_t r, uint32_t k, uint32_t nneg,
                                            float* snap, const SgdParams& p, float alpha, uint64_t idx,
                                            uint32_t epoch, uint32_t seg_lo, uint32_t seg_n) {
@@ -337,7 +338,11 @@ __device__ __forceinline__ void fired_edge(float (&cur)[DIM], uint32_t r, uint32
 #pragma unroll
   for (int d = 0; d < DIM; ++d) { const float df = cur[d] - o[d]; ds += df * df; }
   float g[DIM];
-  if constexpr (GEN) {
+  if constexpr (FUSED) {
+    attract<DIM>(cur, o, g, p, alpha);
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) cur[d] += g[d];
+  } else if constexpr (GEN) {
     // head += clip(c * grad) alpha; tail += clip(c * rev_grad) alpha with rev_grad = -grad
     float den;
     const float gc = metric_coeff(ds, a, p.two_b, p.two_b, -1.0f, &den);
@@ -366,6 +371,10 @@ __device__ __forceinline__ void fired_edge(float (&cur)[DIM], uint32_t r, uint32
     for (int q = 0; q < NEG_BATCH; ++q) {
       if (q0 + q >= nneg) break;
       if (kk[q] == r) continue;
+      if constexpr (FUSED) {
+        repel<DIM>(cur, ob[q], p, alpha);
+        continue;
+      }
       if constexpr (DIM == 2 && !GEN) {
         // the same operations as the generic-DIM code below, two columns per instruction
         const uint64_t c2 = pk2(cur[0], cur[1]);
@@ -482,7 +491,7 @@ __global__ void __launch_bounds__(256, MINB) sgd_epoch_kernel2(
         if (t == j) en = win[t];
       const uint32_t nneg = negatives_at(n, en.y, p.neg_rate);
       const uint64_t idx = LM ? base + (uint64_t)lane * width + ebase + j : base + (uint64_t)(ebase + j) * 32 + lane;
-      fired_edge<DIM, GEN, NEG_BATCH>(cur, r, en.x, nneg, snap, p, alpha, idx, epoch, seg_lo, seg_n);
+      fired_edge<DIM, GEN, NEG_BATCH, false>(cur, r, en.x, nneg, snap, p, alpha, idx, epoch, seg_lo, seg_n);
     }
   }
   if (active) {
@@ -541,7 +550,7 @@ __global__ void __launch_bounds__(256, MINB_DRAM) sgd_epoch_dram(
       const uint64_t idx = first + (uint64_t)(ebase + __ffs(mask) - 1) * 32;
       mask &= mask - 1;
       if (mask) nx = __ldg(lent + (uint64_t)(ebase + __ffs(mask) - 1) * 32);
-      fired_edge<DIM, false, NB_DRAM>(cur, r, en.x, negatives_at(epoch, en.y, p.neg_rate), snap, p, alpha, idx, epoch,
+      fired_edge<DIM, false, NB_DRAM, true>(cur, r, en.x, negatives_at(epoch, en.y, p.neg_rate), snap, p, alpha, idx, epoch,
                                       0u, p.n_vertices);
     }
   }
@@ -686,7 +695,7 @@ __global__ void __launch_bounds__(POOL_BT, MINB_POOL) sgd_epoch_pool(
             e = (uint32_t)__ffs(m) - 1;
             nx = __ldg(lent + e);
           }
-          fired_edge<DIM, GEN, NB_POOL>(cur, row, en.x, negatives_at(epoch, en.y, p.neg_rate), snap, p, alpha, idx,
+          fired_edge<DIM, GEN, NB_POOL, false>(cur, row, en.x, negatives_at(epoch, en.y, p.neg_rate), snap, p, alpha, idx,
                                         epoch, seg_lo, seg_n);
         }
       } else {
