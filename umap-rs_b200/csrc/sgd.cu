@@ -1652,9 +1652,11 @@ void launch_epoch(void (*k)(P...), unsigned grid, unsigned bt, bool overlap, cud
 }
 
 // The launch may overlap the end of the epoch before it (`overlap`): the pooled kernel evaluates its
-// schedule before grid_wait.  A large launch is released to the next one when its last blocks start
-// (2M points: 474 against 484 us per epoch), a smaller one at its blocks' end, since the next epoch's
-// early blocks would fill the SMs unevenly (20k points: 19.2 against 28.6 us, 70k: 34 against 41).
+// schedule before grid_wait.  A large launch is released to the next one when its last blocks start, a
+// smaller one at its blocks' end, since the next epoch's early blocks would fill the SMs unevenly
+// (us per epoch, released at the end / early: 70k points 30.3 / 36.5, 300k (2,400 blocks) 84.0 / 85.2, 500k
+// (3,900) 131.3 / 128.0, 1M 244.4 / 238.0, 2M 472.8 / 469.4).
+constexpr unsigned EARLY_BLOCKS = 3500;
 void sgd_epoch(const SgdLayout& L, float* live, float* snap, const SgdParams& p, uint32_t epoch, float alpha,
                bool overlap, cudaStream_t s) {
   if (L.n_slices == 0) return;
@@ -1669,7 +1671,7 @@ void sgd_epoch(const SgdLayout& L, float* live, float* snap, const SgdParams& p,
                     p, epoch, alpha
   auto pooled = [&](auto k) {
     const unsigned g = blocks(tasks, POOL_BT);
-    launch_epoch(k, g, POOL_BT, overlap, s, UB_SGD_ARGS, g > 8000u);
+    launch_epoch(k, g, POOL_BT, overlap, s, UB_SGD_ARGS, g > EARLY_BLOCKS);
   };
   const bool gen = p.generic_metric;
   auto variants = [&](auto dims) {  // dims(generic rule, batch)
