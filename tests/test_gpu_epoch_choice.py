@@ -93,3 +93,30 @@ def test_batch_kernels_draw_the_same_negatives(ub, monkeypatch, a, b, dim, neg):
             opt.step_epochs(1)
         out.append(opt.embedding())
     assert np.abs(out[0] - out[1]).max() <= 1e-4
+
+
+@pytest.mark.parametrize("kernel", ["lane", "pool", "dram"])
+def test_forced_kernels_quality_with_split_rows(ub, oracle, monkeypatch, kernel):
+    """The 20,000-point sheet-initialised roll of test_embedding_quality_on_a_structured_manifold, in a renamed layout
+    whose rows of more than 16 edges are cut: recall and fuzzy cross-entropy in the oracle's band."""
+    from test_gpu_parity import _assert_quality, _oracle_scores
+    from umap_b200 import quality as Q
+    from umap_b200 import workloads as W
+    X, t = W.swiss_roll(20000, seed=3)
+    idx, dist = W.knn_exact_numpy(X, 15)
+    init = np.stack([t, X[:, 1]], 1).astype(np.float32)
+    cfg = ub.UmapConfig()
+    cfg.optimization.n_epochs = 200
+    rec_o, ce_o, (head, tail, w), (a, b) = _oracle_scores(oracle, idx, dist, init, 200)
+    monkeypatch.setenv("UMAP_B200_SGD_KERNEL", kernel)
+    monkeypatch.setenv("UMAP_B200_RELABEL", "1")
+    res = []
+    for seed in (1, 2, 3):
+        opt = ub.Optimizer(ub.Umap(cfg).learn_manifold(20000, idx, dist), init, 200, cfg)
+        assert {"lane": "kernel2"}.get(kernel, kernel) in opt.layout()["kernel"] and opt.layout()["renamed"]
+        assert opt.tuning()[0] == 16 and np.bincount(head).max() > 16
+        opt.set_seed(seed)
+        opt.step_epochs(200)
+        e = opt.embedding()
+        res.append((Q.knn_recall(e, idx), Q.fuzzy_cross_entropy(e, head, tail, w, a, b)))
+    _assert_quality(res, rec_o, ce_o, f"roll 20k, {kernel}")
