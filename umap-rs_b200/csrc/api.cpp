@@ -586,9 +586,8 @@ void step_epochs_impl(umap_optimizer& o, uint64_t n_ep, int output_metric = UMAP
   UB_CUDA(cudaEventCreate(&ev[0]));
   UB_CUDA(cudaEventCreate(&ev[1]));
   // One launch per epoch, each with its own epoch and learning rate.  The launches are queued while
-  // earlier epochs run (about 2 us of host time each, an epoch takes 10 us and more); a CUDA graph of
-  // the loop costs its capture and instantiation before the first epoch starts (500 points, 500
-  // epochs: 9.0 ms a fit with one, 6.7 ms without).
+  // earlier epochs run (about 2 us of host time each, an epoch takes 14 us and more); a CUDA graph of
+  // the loop costs its capture and instantiation before the first epoch starts.
   UB_CUDA(cudaEventRecord(ev[0], s));
   for (uint64_t epoch = o.current_epoch; epoch < o.current_epoch + n_ep; ++epoch) {
     const float alpha = o.initial_alpha * (1.0f - ((float)epoch / (float)o.total_epochs));  // :317

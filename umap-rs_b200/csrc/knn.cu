@@ -538,7 +538,7 @@ __global__ void __launch_bounds__(KNN_THREADS, 1) knn_candidates_kernel(
     // epilogue: warps 2..9; warp w owns tensor-memory lane quarter w % 4 (query rows) and half
     // (w - 2) / 4 of each tile's columns, with its own list per row: entries below the row's
     // threshold go to free slots, and a list that runs out of them is reduced to its HC smallest
-    // (reduce_lists), which lowers the threshold.
+    // (thin_list), which lowers the threshold.
     const int q = warp & 3, half = (warp - 2) >> 2;
     const int trow = q * 32 + lane;
     float* ld = lists + half * CAP * QM + trow;

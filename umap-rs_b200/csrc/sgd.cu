@@ -578,7 +578,9 @@ __global__ void __launch_bounds__(256, MINB_DRAM) sgd_epoch_dram(
 // Small graphs are bound by the chain of one task's firings - row loads, then 6 dependent updates -
 // with the chip half empty.  Drawing a firing's rows during the loads of the one before took the
 // generator out of it (500 points 18.6 -> 14.3 us per epoch, 10k 21.3 -> 17.5, 70k 31.0 -> 28.4, 2M
-// 456 -> 439; a lane per task: 27, 33, 40, 630).  Loading the rows themselves one firing ahead, with
+// 456 -> 439, in 100 epochs at small rates).  At rate 1, this kernel / a lane per task, us per epoch: 500
+// points 17.2 / 31.5, 10k 18.7 / 32.4, 70k 29.9 / 39.6, 300k 84 / 106, 1M 245 / 304, 2M 466 / 581 (494 on
+// average over 500 epochs, at the power limit).  Loading the rows themselves one firing ahead, with
 // 8 lanes per task, ran 500 points in 11 us and no larger set faster than this, but its updates
 // see older rows, and layouts of some thousand points moved by more than two runs differ.
 // `early` lets the next epoch's blocks start as soon as this launch's last ones have, otherwise at
@@ -1453,8 +1455,8 @@ bool lane_major_entries(uint64_t n, bool segmented, EpochKernel kernel) {
 
 // Whether a plain fit's layout renames its vertices into a locality order (order.cu): from the
 // sizes at which random rows of the caller's order mostly miss L2.
-// UMAP_B200_RELABEL=0 / 1 forces either.  The generic-metric rule never renames (its caller
-// passes rename = false): it is sensitive to which rows update at the same time (its split
+// UMAP_B200_RELABEL=0 / 1 forces either.  The generic-metric rule never renames
+// (build_sgd_layout): it is sensitive to which rows update at the same time (its split
 // rows showed that), and its parity with the reference was established in the caller's order;
 // on a 6,000-point roll one renamed run sat 2.6% from a plain one, inside that small case's
 // run-to-run spread, so renaming is not shown to move it, only not shown to be harmless.

@@ -74,8 +74,9 @@ __device__ __forceinline__ bool mbar_wait(uint32_t addr, uint32_t phase) {
 }
 
 // Programmatic dependent launch.  `grid_wait` returns once every grid this launch depends on
-// has completed and its memory is visible (a no-op for a launch without the attribute); a
-// kernel reads and writes no global memory, and allocates no tensor memory, before it.
+// has completed and its memory is visible (a no-op for a launch without the attribute).  Before it a
+// kernel allocates no tensor memory and touches no global memory, but for reads of what was complete
+// before the first launch of the chain that has no such attribute (the pooled epoch's layout arrays).
 // `grid_release` lets the dependent launch be scheduled once every CTA of this grid has
 // executed it (or exited); the dependent's own `grid_wait` still waits for this grid's end.
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
