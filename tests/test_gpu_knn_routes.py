@@ -30,6 +30,16 @@ def test_alternating_classes(ub, oracle, n, classes, k):
     assert rec < n // 20
 
 
+@pytest.mark.parametrize("n,d,k", [(10000, 256, 100), (4096, 8, 64)])
+def test_ordered_rows(ub, oracle, n, d, k):
+    """Points along a line in their order: the 2 S rows next to one another go to as many lists, so none overflows."""
+    X = np.repeat(np.arange(n, dtype=np.float32)[:, None], d, axis=1)
+    gi, gd, rec = ub.knn_bruteforce(X, k, return_stats=True)
+    oi, od = oracle.knn_bruteforce(X, k, rows=(0, 200))
+    assert np.array_equal(gi[:200], oi) and np.array_equal(gd[:200], od)
+    assert rec < n // 100
+
+
 @pytest.mark.parametrize("n,d,k,rows", [(3000, 12, 10, 128), (2500, 20, 25, 1024), (2600, 8, 100, 640), (20001, 6, 15, 4096),
                                         (17000, 5, 50, 3072), (2304, 9, 15, 2176), (2049, 9, 15, 2176)])
 def test_rows_in_several_passes(ub, monkeypatch, n, d, k, rows):

@@ -1046,40 +1046,26 @@ __global__ void knn_exact_merge_kernel(const uint64_t* __restrict__ part, const 
   }
 }
 
-// Position p of the scan order takes the rank of the locality order that deals consecutive ranks round-robin over the 2 S lists of a group of S tiles, so a row's
-// neighbours, which are near in rank, spread evenly over its lists.  Groups are S whole tiles, then
-// one of the whole tiles left; rows past them keep their rank.
+// Position p of the scan order takes the rank of the locality order (or of the caller's order, perm null) that
+// deals each run of 2 S consecutive ranks over the 2 S lists of a group of S tiles, one to a list: a row's
+// neighbours, which are near in rank, spread evenly over its lists.  Every run is dealt from another list on
+// (a hash of the run), or ranks at a distance of 2 S would all meet in one list: 8,000 rows in 16
+// alternating classes, k = 100, had every row recomputed, 21.2 ms against 3.9 for the same rows shuffled.
+// Groups are S whole tiles, then one of the whole tiles left; rows past them keep their rank.
 __global__ void deal_ranks_kernel(const uint32_t* __restrict__ perm, int64_t n, int S, uint32_t* __restrict__ out) {
   const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= n) return;
   const int64_t whole = n / DBN, g = p / DBN / S;  // whole tiles, this position's group
-  const int64_t tiles = min((int64_t)S, whole - g * S);
+  const uint32_t lists = 2u * (uint32_t)min((int64_t)S, whole - g * S);
   int64_t rank = p;
   if (p < whole * DBN) {
-    const int64_t first = g * S * DBN, t = (p - first) / DBN, in = p % DBN;
-    rank = first + (in % (DBN / 2)) * (2 * tiles) + 2 * t + in / (DBN / 2);
+    const int64_t first = g * S * DBN;
+    const uint32_t at = (uint32_t)(p - first), run = at % (DBN / 2), list = at / (DBN / 2);
+    uint32_t h = ((uint32_t)g * (DBN / 2) + run) * 0x9E3779B1u;
+    h = (h ^ (h >> 16)) * 0x85EBCA6Bu;
+    rank = first + run * lists + (list + ((h >> 16) & 0xFFu)) % lists;
   }
-  out[p] = perm[rank];
-}
-
-// Long lists of sets without a locality order: position p takes a scattered row, so that a row's neighbours
-// spread over its lists whatever the caller's order.  (Dealt like a locality order, 8,000 rows whose
-// 16 classes alternate had every neighbour of a row in one list: all rows recomputed, 21.2 ms against
-// 3.9 for the same rows shuffled.)  A bijection of b-bit numbers - odd multiply, add, xor with its own high
-// half, three times - repeated until it lands below n; 2^b < 2n, so mostly once or twice.
-__global__ void scatter_ranks_kernel(uint32_t n, int bits, uint32_t* __restrict__ out) {
-  const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= n) return;
-  const uint32_t mask = (1u << bits) - 1u;
-  uint32_t x = p;
-  do {
-#pragma unroll
-    for (int r = 0; r < 3; ++r) {
-      x = (x * 0x9E3779B1u + 0x7F4A7C15u) & mask;
-      x ^= x >> ((bits + 1) / 2);
-    }
-  } while (x >= n);
-  out[p] = x;
+  out[p] = perm ? perm[rank] : (uint32_t)rank;
 }
 
 inline unsigned blocks_for(int64_t n, unsigned bt) { return (unsigned)std::min<int64_t>((n + bt - 1) / bt, 1 << 20); }
@@ -1115,8 +1101,7 @@ void exact_rows(const float* X, int64_t n, int d, int k, const uint32_t* rows, u
 //  * k <= KNN_MAX_K: the count with the least ceil(items / SMs) * (T + 46 ln(T + 1)) for T tiles per item:
 //    an item's entries, which come with the logarithm of its columns, cost 46 tiles per e-fold.
 //    For k > 16 and fewer query blocks than SMs at least two, for 4 candidates per neighbour.
-//  * Longer lists: a row's neighbours fall evenly on the splits' lists (deal_ranks_kernel,
-//    scatter_ranks_kernel), each of which
+//  * Longer lists: a row's neighbours fall evenly on the splits' lists (deal_ranks_kernel), each of which
 //    keeps HC = 32: 4 splits up to k = 64, else 8, for at most 8 of the k on average (the points within
 //    the error margin of the k-th come on top).  A row whose list overflows fails its certificate and
 //    is recomputed exactly.
@@ -1276,10 +1261,8 @@ KnnStats knn_bruteforce(const float* X, uint64_t n, uint64_t d, uint64_t k, uint
     UB_LAUNCH_CHECK();
     st.reordered = 1;
   } else if (k > (uint64_t)KNN_MAX_K) {
-    int bits = 1;
-    while ((1ull << bits) < n) ++bits;
     perm.alloc(n, s);
-    scatter_ranks_kernel<<<blocks_for((int64_t)n, 256), 256, 0, s>>>((uint32_t)n, bits, perm.p);
+    deal_ranks_kernel<<<blocks_for((int64_t)n, 256), 256, 0, s>>>(nullptr, (int64_t)n, S, perm.p);
     UB_LAUNCH_CHECK();
   }
   knn_prep_kernel<<<prep_grid, 256, 0, s>>>(X, (int64_t)n, di, (int)dp, n_pad, mean.p, scale, perm.p, xh.p, nb.p, nullptr,
