@@ -50,3 +50,16 @@ def test_rows_in_several_passes(ub, monkeypatch, n, d, k, rows):
     monkeypatch.setenv("UMAP_B200_KNN_ROWS", str(rows))
     got = ub.knn_bruteforce(X, k)
     assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
+
+
+@pytest.mark.parametrize("n,d,k,classes,sep", [(8000, 1024, 15, 50, 10), (10000, 256, 15, 50, 10), (12000, 784, 5, 10, 5),
+                                               (6000, 784, 30, 50, 10)])
+def test_wide_clusters_pass_their_certificates(ub, oracle, n, d, k, classes, sep):
+    """Clusters so far apart that the error margin of a row holds more points than one or two lists: the splits'
+    lists together hold them, and few rows are recomputed."""
+    g = np.random.Generator(np.random.PCG64(n))
+    X = (g.standard_normal((n, d)) + sep * g.standard_normal((classes, d))[g.integers(0, classes, n)]).astype(np.float32)
+    gi, gd, rec = ub.knn_bruteforce(X, k, return_stats=True)
+    oi, od = oracle.knn_bruteforce(X, k, rows=(0, 100))
+    assert np.array_equal(gi[:100], oi) and np.array_equal(gd[:100], od)
+    assert rec < n // 10

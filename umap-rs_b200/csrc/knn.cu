@@ -268,7 +268,8 @@ __device__ __forceinline__ void tmem_read(uint32_t (&r)[16], uint32_t taddr) {
 //    row's k-th smallest is at most y, and only entries under y plus the error margin can matter
 //    (Margin): the threshold follows every hit.
 //  * a list whose slots run out keeps what is at or below the threshold, and of that the HC smallest
-//    (thin_list; the whole warp at once, a lane per list).  Longer k have only this (RL = 0).
+//    (thin_list; the whole warp at once, a lane per list).  Longer k have only this (RL = 0), and keep
+//    HC - 4 to HC, which is found sooner.
 // Nothing moves: the slots of the others become free, and tau falls to a bound that no entry left
 // out, now or later, is below.
 struct Margin {
@@ -286,7 +287,7 @@ struct ListState {
   uint32_t occ0, occ1;
   float tau;
 };
-__device__ __noinline__ ListState thin_list(const float* ld, uint32_t occ0, uint32_t occ1, float tau, float mn) {
+__device__ __noinline__ ListState thin_list(const float* ld, uint32_t occ0, uint32_t occ1, float tau, float mn, int keep) {
   float e[CAP];  // free slots count as infinite
 #pragma unroll
   for (int j = 0; j < CAP; ++j) {
@@ -332,7 +333,7 @@ __device__ __noinline__ ListState thin_list(const float* ld, uint32_t occ0, uint
   float l = mn;
   const bool cut = have > HC;
   if (__any_sync(0xFFFFFFFFu, cut)) {
-    const float x = search(cut, HC - 4, HC, l, top, have);
+    const float x = search(cut, keep, HC, l, top, have);
     if (cut) t = x;
   }
   uint32_t m0 = 0, m1 = 0;
@@ -572,7 +573,7 @@ __global__ void __launch_bounds__(KNN_THREADS, 1) knn_candidates_kernel(
 #pragma unroll
       for (int i = 0; i < RL; ++i) best[i] = i < RL - rank ? -INFINITY : INFINITY;
       auto thin = [&]() {
-        const ListState st = thin_list(ld, occ0, occ1, tau, mn);
+        const ListState st = thin_list(ld, occ0, occ1, tau, mn, RL ? HC : HC - 4);
         occ0 = st.occ0;
         occ1 = st.occ1;
         tau = st.tau;
@@ -1098,9 +1099,13 @@ void exact_rows(const float* X, int64_t n, int d, int k, const uint32_t* rows, u
 
 // Database splits of the candidate pass (0: the exact path).  Every (query block, split) pair is one
 // work item of a persistent CTA, and every split keeps NCAND candidates per row in two lists of HC.
-//  * k <= KNN_MAX_K: the count with the least ceil(items / SMs) * (T + 46 ln(T + 1)) for T tiles per item:
-//    an item's entries, which come with the logarithm of its columns, cost 46 tiles per e-fold.
-//    For k > 16 and fewer query blocks than SMs at least two, for 4 candidates per neighbour.
+//  * k <= KNN_MAX_K: halvings of the database until every SM has an item, or 2 tiles are left; three splits
+//    instead of two where they take no more waves of items (10,000 x 32, k = 15: 0.62 ms with two, 0.56 with
+//    three; with one, whose items are longer but fill one wave, 0.55).  No fewer: a row whose error margin holds
+//    more points than its lists (clusters far apart in many dimensions) fails its certificate and is computed
+//    again, 20.5 ms for 10,000 x 256 in 50 clusters with one split, 8,587 rows, against 1.0 with three.  And no
+//    more: every candidate within the margin is one more exact distance (5,000 x 784 in 10 clusters, k = 10: 1.5
+//    ms with four, 2.1 with six).
 //  * Longer lists: a row's neighbours fall evenly on the splits' lists (deal_ranks_kernel), each of which
 //    keeps HC = 32: 4 splits up to k = 64, else 8, for at most 8 of the k on average (the points within
 //    the error margin of the k-th come on top).  A row whose list overflows fails its certificate and
@@ -1113,20 +1118,10 @@ int pick_splits(uint64_t n, uint64_t k, int64_t q_blocks, int64_t tiles, int sms
     if (n < LONG_LIST_MIN) return 0;
     return k <= 64 ? 4 : 8;
   }
-  const int counts[] = {1, 2, 3, 4, 6, 8};
-  int best = 1;
-  double cost = INFINITY;
-  for (int S : counts) {
-    if (S > 1 && tiles / S < 2) break;
-    if (S == 1 && k > 16 && q_blocks < sms && tiles >= 4) continue;
-    const double T = (double)tiles / S;
-    const double c = (double)((q_blocks * S + sms - 1) / sms) * (T + 46.0 * std::log(T + 1.0));
-    if (c < cost) {
-      cost = c;
-      best = S;
-    }
-  }
-  return best;
+  int S = 1;
+  while (S < 8 && q_blocks * S < sms && tiles / (2 * S) >= 2) S *= 2;
+  const auto waves = [&](int s) { return (q_blocks * s + sms - 1) / sms; };
+  return S == 2 && tiles >= 6 && waves(3) == waves(2) ? 3 : S;
 }
 
 // Rows whose candidates a call holds at once (a multiple of QM): 512 bytes a row and split, so that the
