@@ -844,6 +844,10 @@ __global__ void __launch_bounds__(RERANK_BT) knn_rerank_kernel(
       lo = fminf(lo, __shfl_xor_sync(0xFFFFFFFFu, lo, o));
       hi = fmaxf(hi, __shfl_xor_sync(0xFFFFFFFFu, hi, o));
     }
+    float tau = lane < 2 * S ? tau_in[w * 2 * S + lane] : INFINITY;  // (split, half)
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) tau = fminf(tau, __shfl_xor_sync(0xFFFFFFFFu, tau, o));
+    const float lb = tau < INFINITY ? distance_lower_bound(tau, xr, R, gamma, scale, d, dp) : INFINITY;
     float U = INFINITY;
     if (have > k) {
       // hi: at least k candidates at or below it, close to the k-th
@@ -859,6 +863,13 @@ __global__ void __launch_bounds__(RERANK_BT) knn_rerank_kernel(
         } else {
           lo = mid;
         }
+      }
+      // The k-th approximate distance, above lo, is at the certificate's bound or beyond: the exact one, which
+      // the bound's margins stand far from, will not pass either, and the row is not worth evaluating
+      // (3,000 x 784 of very uneven lengths, k = 128, all rows failing: 24.7 -> 23.0 ms a call).
+      if (sqrtf(fmaxf(lo, 0.0f)) / scale >= lb) {
+        if (lane == 0) fail_rows[atomicAdd(fail_count, 1u)] = (uint32_t)row;
+        continue;
       }
       U = distance_upper_bound(hi, xr, R, gamma, scale, d, dp);
     }
@@ -905,15 +916,8 @@ __global__ void __launch_bounds__(RERANK_BT) knn_rerank_kernel(
       }
       last = wm;
     }
-    if (lane == 0) {
-      float tau = INFINITY;
-      for (int s = 0; s < 2 * S; ++s) tau = fminf(tau, tau_in[w * 2 * S + s]);  // (split, half)
-      if (tau < INFINITY) {
-        const float lb = distance_lower_bound(tau, xr, R, gamma, scale, d, dp);
-        if (last == ~0ull || !(__uint_as_float((uint32_t)(last >> 32)) < lb))
-          fail_rows[atomicAdd(fail_count, 1u)] = (uint32_t)row;
-      }
-    }
+    if (lane == 0 && tau < INFINITY && (last == ~0ull || !(__uint_as_float((uint32_t)(last >> 32)) < lb)))
+      fail_rows[atomicAdd(fail_count, 1u)] = (uint32_t)row;
   }
 }
 
