@@ -679,7 +679,7 @@ std::unique_ptr<umap_fitted> fit_impl(const umap_config& c, uint64_t n_samples, 
 }
 
 // ------------------------------------------------------------------ autotuning
-// Picks the SGD task length ("edges per thread") and the lane kernel's block shape by timing two
+// Picks the SGD task length ("edges per thread") and, for the kernels that take any, the block shape by timing two
 // epochs of each candidate on a scratch copy of the embedding.  Choices are cached per
 // problem size (vertices, edges in MiB units, dims) and kernel for the life of the process; one
 // whose search ended at a task length that holds every row stands for batches with rows as short.
@@ -732,7 +732,7 @@ void tune_layout(umap_optimizer& o, const KeptEdges& K) {
     const uint32_t own = L.block_threads;
     bool better = false;
     for (uint32_t bt : {128u, 256u}) {
-      if (bt != own && L.kernel != EpochKernel::Lane) continue;
+      if (bt != own && L.kernel != EpochKernel::Lane && L.kernel != EpochKernel::AnyDim) continue;
       L.block_threads = bt;
       sgd_epoch(L, scratch.p, scratch.p + n * o.dim, p, mid, 0.5f, false, s);  // warm-up
       UB_CUDA(cudaEventRecord(e0, s));

@@ -1726,8 +1726,8 @@ void sgd_epoch(const SgdLayout& L, float* live, float* snap, const SgdParams& p,
       launch_epoch(p.dim == 1 ? sgd_epoch_dram<1> : sgd_epoch_dram<2>, blocks(tasks, BT), BT, false, s, UB_SGD_ARGS);
       break;
     case EpochKernel::AnyDim:
-      launch_epoch(gen ? sgd_epoch_anydim<true> : sgd_epoch_anydim<false>, blocks(tasks, BT), BT, false, s, UB_SGD_ARGS,
-                   L.lane_major);
+      launch_epoch(gen ? sgd_epoch_anydim<true> : sgd_epoch_anydim<false>, blocks(tasks, L.block_threads),
+                   L.block_threads, false, s, UB_SGD_ARGS, L.lane_major);
       break;
   }
 #undef UB_SGD_ARGS
