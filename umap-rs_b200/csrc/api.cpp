@@ -863,8 +863,8 @@ std::unique_ptr<umap_optimizer> batch_new_impl(const umap_config& c, uint64_t n_
     KeptEdges K;
     compute_kept_edges(*o, K, true, true);
     const char* tune = getenv("UMAP_B200_AUTOTUNE");
-    if ((tune && tune[0] == '0') || total_epochs < 2) build_sgd_layout(K.ptr.p, K.tail.p, K.eps.p, N, (uint32_t)dims, 0, false, o->initial_alpha,
-                                                    o->layout, s, &so);
+    if ((tune && tune[0] == '0') || total_epochs < 2)
+      build_sgd_layout(K.ptr.p, K.tail.p, K.eps.p, N, (uint32_t)dims, 0, false, o->initial_alpha, o->layout, s, &so);
     else tune_layout(*o, K);
   }
   set_l2_window(*o, true);
