@@ -254,38 +254,41 @@ __device__ __forceinline__ float square_ftz(const float (&df)[DIM]) {
   for (int d = 0; d < DIM; ++d) ds = fmaf(df[d], df[d], ds);
   return ds;
 }
-// Attraction coefficient -2ab ds^b / (ds (a ds^b ds + 1)), of square_ftz's distance.
-__device__ __forceinline__ float attract_coeff(float ds, const SgdParams& p) {
-  const float pb = ftz_exp2(p.b * ftz_log2(ds));
-  const float c = (p.neg_attr * pb) * ftz_rcp(fmaf(p.a * ds * ds, pb, ds));
-  return ds > FLT_MIN ? c : 0.0f;
-}
-// 1 / ((0.001 + ds)(a ds^b ds + 1)), the repulsion coefficient over 2 gamma b.
-__device__ __forceinline__ float repel_inv(float ds, const SgdParams& p) {
-  const float u = 0.001f + ds, v = u * (p.a * ds);
-  return ftz_rcp(fmaf(v, ftz_exp2(p.b * ftz_log2(ds)), u));
-}
-// Attractive move g of the head row (the tail gets -g).
+// Attractive move g of the head row (the tail gets -g): coefficient -2ab ds^b / (ds (a ds^b ds + 1)).  What keeps
+// the rule's limits stands beside the chain from the distance to the reciprocal: a NaN distance counts as 0,
+// whose coefficient is 0, and where the denominator overflows the row's difference is left out of the
+// product, which could overflow before the reciprocal's 0 meets it.
 template <int DIM>
 __device__ __forceinline__ void attract(float (&cur)[DIM], const float (&o)[DIM], float (&g)[DIM], const SgdParams& p,
                                         float alpha) {
   float df[DIM];
 #pragma unroll
   for (int d = 0; d < DIM; ++d) df[d] = cur[d] - o[d];
-  const float c = attract_coeff(square_ftz<DIM>(df), p);
+  const float sq = square_ftz<DIM>(df), ds = fmaxf(sq, FLT_MIN);
+  const float pb = ftz_exp2(p.b * ftz_log2(ds)), den = fmaf(p.a * ds * ds, pb, ds), inv = ftz_rcp(den);
+  const float num = sq > FLT_MIN ? p.neg_attr * pb : 0.0f;
+  const bool far = !(den <= FLT_MAX);
 #pragma unroll
-  for (int d = 0; d < DIM; ++d) g[d] = clip4(c * df[d]) * alpha;
+  for (int d = 0; d < DIM; ++d) g[d] = clip4((num * (far ? 0.0f : df[d])) * inv) * alpha;
 }
-// Repulsive move from row o.
+// Repulsive move from row o: coefficient 2 gamma b / ((0.001 + ds)(a ds^b ds + 1)), where it is above 0; the
+// denominator's range tells beside its reciprocal.  `rep` = max(2 gamma b, 0).
 template <int DIM>
-__device__ __forceinline__ void repel(float (&cur)[DIM], const float (&o)[DIM], const SgdParams& p, float alpha) {
-  float df[DIM];
+__device__ __forceinline__ bool repel_move(const float (&df)[DIM], float (&g)[DIM], const SgdParams& p, float rep) {
+  const float ds = square_ftz<DIM>(df), u = 0.001f + ds, v = u * (p.a * ds);
+  const float den = fmaf(v, ftz_exp2(p.b * ftz_log2(ds)), u), inv = ftz_rcp(den);
+#pragma unroll
+  for (int d = 0; d < DIM; ++d) g[d] = clip4((rep * df[d]) * inv);
+  return den > 0.0f && den <= FLT_MAX;
+}
+template <int DIM>
+__device__ __forceinline__ void repel(float (&cur)[DIM], const float (&o)[DIM], const SgdParams& p, float rep, float alpha) {
+  float df[DIM], g[DIM];
 #pragma unroll
   for (int d = 0; d < DIM; ++d) df[d] = cur[d] - o[d];
-  const float inv = repel_inv(square_ftz<DIM>(df), p);
-  if (p.pos_rep * inv > 0.0f) {
+  if (repel_move<DIM>(df, g, p, rep)) {
 #pragma unroll
-    for (int d = 0; d < DIM; ++d) cur[d] = fmaf(clip4((p.pos_rep * df[d]) * inv), alpha, cur[d]);
+    for (int d = 0; d < DIM; ++d) cur[d] = fmaf(g[d], alpha, cur[d]);
   }
 }
 
@@ -298,7 +301,7 @@ template <int DIM, bool GEN, int NEG_BATCH, bool FUSED>
 __device__ __forceinline__ void fired_edge(float (&cur)[DIM], uint32_t r, uint32_t k, uint32_t nneg,
                                            float* snap, const SgdParams& p, float alpha, uint64_t idx,
                                            uint32_t epoch, uint32_t seg_lo, uint32_t seg_n) {
-  const float a = p.a, b = p.b;
+  const float a = p.a, b = p.b, rep = fmaxf(p.pos_rep, 0.0f);
   float* oth = snap + (uint64_t)k * DIM;
   float o[DIM];
   load_row<DIM>(o, oth);
@@ -372,7 +375,7 @@ __device__ __forceinline__ void fired_edge(float (&cur)[DIM], uint32_t r, uint32
       if (q0 + q >= nneg) break;
       if (kk[q] == r) continue;
       if constexpr (FUSED) {
-        repel<DIM>(cur, ob[q], p, alpha);
+        repel<DIM>(cur, ob[q], p, rep, alpha);
         continue;
       }
       if constexpr (DIM == 2 && !GEN) {
@@ -583,15 +586,21 @@ __global__ void __launch_bounds__(256, MINB_DRAM) sgd_epoch_dram(
 // average over 500 epochs, at the power limit).  Loading the rows themselves one firing ahead, with
 // 8 lanes per task, ran 500 points in 11 us and no larger set faster than this, but its updates
 // see older rows, and layouts of some thousand points moved by more than two runs differ.
+// MANY: rates whose firings draw more negatives than are fetched together (NB_POOL or more a sample) fetch them as many
+// at a time, too, and draw the next firing's rows after that (20k points, 60 epochs, 20 / 50 negatives a sample:
+// 7.5 / 17.2 ms a fit with one row after another, 4.4 / 8.2 so, a lane per task 6.6 / 13.5).  Lower rates lose by the
+// later draw (us per epoch without / with, 20k points: 5 a sample 18.8 / 19.6, 7 29.6 / 28.8, 8 36.4 / 31.4;
+// 300k: 79.6 / 80.1, 100.2 / 103.1, 116.4 / 116.4).
 // `early` lets the next epoch's blocks start as soon as this launch's last ones have, otherwise at
 // its end (see sgd_epoch).
 constexpr int POOL_WIN = 32;
-template <int DIM, bool GEN, bool SEG>
+template <int DIM, bool GEN, bool SEG, bool MANY>
 __global__ void __launch_bounds__(POOL_BT, MINB_POOL) sgd_epoch_pool(
     const uint64_t* __restrict__ slice_base, const uint32_t* __restrict__ slice_width,
     const uint32_t* __restrict__ split_mask, const uint32_t* __restrict__ rowid,
     const uint2* __restrict__ entry, uint64_t n_slices, float* __restrict__ live, float* snap,
     SgdParams p, uint32_t epoch, float alpha, bool early) {
+  const float rep = fmaxf(p.pos_rep, 0.0f);
   constexpr int SL = POOL_BT / 32;  // slices: one per warp while the schedule is evaluated
   // Batches take windows in turns of two buffers, so that a warp goes on to the next window's schedule
   // while others still fire (77 -> 75 us per epoch at 64 instances; a plain 70k-point fit 28.8 -> 29.9).
@@ -747,32 +756,40 @@ __global__ void __launch_bounds__(POOL_BT, MINB_POOL) sgd_epoch_pool(
           const uint64_t at = idx;
           if constexpr (!FAR) step();
           more = m != 0;
-          // (a firing of more negatives than fetched together still needs the arrays: the next is drawn after it)
-          if (more && drawn <= NB_POOL) next();
+          // (MANY: a firing of more negatives than fetched together still needs the arrays)
+          if (more && (!MANY || drawn <= NB_POOL)) next();
           attract<DIM>(cur, o, g, p, alpha);
 #pragma unroll
           for (int d = 0; d < DIM; ++d) cur[d] += g[d];
           sub_row<DIM>(oth, g);
 #pragma unroll
           for (int q = 0; q < NB_POOL; ++q)
-            if ((ok >> q) & 1u) repel<DIM>(cur, ob[q], p, alpha);
-          // as many at a time again (20k points, 60 epochs, 20 / 50 negatives a sample: 7.5 / 17.2 ms a fit
-          // with one row after another, 4.6 / 8.8 so; a lane per task 6.7 / 13.4)
-          if (drawn > NB_POOL) {
-            const NegRng rng(p.seed, at, epoch);
-            for (uint32_t q0 = NB_POOL; q0 < drawn; q0 += NB_POOL) {
-              uint64_t rnd = 0;
+            if ((ok >> q) & 1u) repel<DIM>(cur, ob[q], p, rep, alpha);
+          const NegRng rng(p.seed, at, epoch);
+          if constexpr (MANY) {
+            if (drawn > NB_POOL) {
+              for (uint32_t q0 = NB_POOL; q0 < drawn; q0 += NB_POOL) {
+                uint64_t rnd = 0;
 #pragma unroll
-              for (int q = 0; q < NB_POOL; ++q) {
-                if ((q & 1) == 0) rnd = rng.pair((q0 + q) >> 1);
-                kk[q] = q0 + q < drawn ? seg_lo + __umulhi((q & 1) ? (uint32_t)(rnd >> 32) : (uint32_t)rnd, seg_n) : row;
-                if (kk[q] != row) load_row_l2<DIM>(ob[q], snap + (uint64_t)kk[q] * DIM);
+                for (int q = 0; q < NB_POOL; ++q) {
+                  if ((q & 1) == 0) rnd = rng.pair((q0 + q) >> 1);
+                  kk[q] = q0 + q < drawn ? seg_lo + __umulhi((q & 1) ? (uint32_t)(rnd >> 32) : (uint32_t)rnd, seg_n) : row;
+                  if (kk[q] != row) load_row_l2<DIM>(ob[q], snap + (uint64_t)kk[q] * DIM);
+                }
+#pragma unroll
+                for (int q = 0; q < NB_POOL; ++q)
+                  if (kk[q] != row) repel<DIM>(cur, ob[q], p, rep, alpha);
               }
-#pragma unroll
-              for (int q = 0; q < NB_POOL; ++q)
-                if (kk[q] != row) repel<DIM>(cur, ob[q], p, alpha);
+              if (more) next();
             }
-            if (more) next();
+          } else {
+            for (uint32_t q = NB_POOL; q < drawn; ++q) {  // rare: the rate is below NB_POOL
+              const uint64_t rnd = rng.pair(q >> 1);
+              const uint32_t k = seg_lo + __umulhi((q & 1) ? (uint32_t)(rnd >> 32) : (uint32_t)rnd, seg_n);
+              if (k == row) continue;
+              load_row_l2<DIM>(o, snap + (uint64_t)k * DIM);
+              repel<DIM>(cur, o, p, rep, alpha);
+            }
           }
         }
       }
@@ -883,6 +900,7 @@ __global__ void __launch_bounds__(256) sgd_epoch_rows(
     const uint2* __restrict__ entry, uint64_t n_slices, float* __restrict__ live, float* snap,
     SgdParams p, uint32_t epoch, float alpha) {
   constexpr int NB = 6;  // negative rows fetched together
+  const float rep = fmaxf(p.pos_rep, 0.0f);
   const uint64_t slice = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint32_t lane = threadIdx.x & 31;
   if (slice >= n_slices) return;
@@ -951,10 +969,9 @@ __global__ void __launch_bounds__(256) sgd_epoch_rows(
           if (split) load_row_l2<DIM>(cur, hrow);
 #pragma unroll
           for (int d = 0; d < DIM; ++d) df[d] = cur[d] - x[q][d];
-          const float inv = repel_inv(square_ftz<DIM>(df), p);
-          if (!(p.pos_rep * inv > 0.0f)) continue;
+          if (!repel_move<DIM>(df, g, p, rep)) continue;
 #pragma unroll
-          for (int d = 0; d < DIM; ++d) g[d] = clip4((p.pos_rep * df[d]) * inv) * alpha;
+          for (int d = 0; d < DIM; ++d) g[d] *= alpha;
           move(g);
         }
       }
@@ -1694,10 +1711,12 @@ void sgd_epoch(const SgdLayout& L, float* live, float* snap, const SgdParams& p,
   switch (L.kernel) {
     case EpochKernel::Pool: {
       auto dims = [&](auto gen, auto seg) {
-        if (p.dim == 1) pooled(sgd_epoch_pool<1, gen.value, seg.value>);
-        else if (p.dim == 2) pooled(sgd_epoch_pool<2, gen.value, seg.value>);
-        else if (p.dim == 3) pooled(sgd_epoch_pool<3, gen.value, seg.value>);
-        else pooled(sgd_epoch_pool<4, gen.value, seg.value>);
+        constexpr bool G = gen.value, S = seg.value;
+        auto many = [&](auto k, auto k_many) { pooled(!G && p.neg_rate >= (uint32_t)NB_POOL ? k_many : k); };
+        if (p.dim == 1) many(sgd_epoch_pool<1, G, S, false>, sgd_epoch_pool<1, G, S, !G>);
+        else if (p.dim == 2) many(sgd_epoch_pool<2, G, S, false>, sgd_epoch_pool<2, G, S, !G>);
+        else if (p.dim == 3) many(sgd_epoch_pool<3, G, S, false>, sgd_epoch_pool<3, G, S, !G>);
+        else many(sgd_epoch_pool<4, G, S, false>, sgd_epoch_pool<4, G, S, !G>);
       };
       variants(dims);
       break;
