@@ -582,7 +582,7 @@ __global__ void __launch_bounds__(256, MINB_DRAM) sgd_epoch_dram(
 // with the chip half empty.  Drawing a firing's rows during the loads of the one before took the
 // generator out of it (500 points 18.6 -> 14.3 us per epoch, 10k 21.3 -> 17.5, 70k 31.0 -> 28.4, 2M
 // 456 -> 439, in 100 epochs at small rates).  At rate 1, this kernel / a lane per task, us per epoch: 500
-// points 17.2 / 31.5, 10k 18.7 / 32.4, 70k 29.9 / 39.6, 300k 84 / 106, 1M 245 / 304, 2M 466 / 581 (494 on
+// points 15.5 / 30.6, 10k 17.5 / 31.5, 70k 28.6 / 39.2, 300k 83 / 106, 1M 236 / 305, 2M 463 / 582 (495 on
 // average over 500 epochs, at the power limit).  Loading the rows themselves one firing ahead, with
 // 8 lanes per task, ran 500 points in 11 us and no larger set faster than this, but its updates
 // see older rows, and layouts of some thousand points moved by more than two runs differ.
@@ -1442,7 +1442,7 @@ bool small_graph(uint64_t n_slices) {
 //    hold it, 3,000 of 15 do not, 22% of the pairs against 3%), RACING_RATE_WIDE for the rest.
 //    Renamed layouts take Pool at every rate: their locality order alone moves two runs as far apart as
 //    the kernels (5M points: 7.2e-3 either way).
-//    Time, Lane / Pool, ms per fit: 10k points 7.3 / 4.4, 70k 9.1 / 6.9, 1M 35.4 / 28.2, 64 instances
+//    Time, Lane / Pool, ms per fit: 10k points 7.3 / 4.3, 70k 9.1 / 6.9, 1M 35.4 / 28.2, 64 instances
 //    23.6 / 16.7; AnyDim / Rows, 20k points in 5-D 50 / 11.
 // UMAP_B200_SGD_KERNEL=lane / pool / dram / rows / any forces one that can run the layout.
 constexpr float RACING_RATE = 0.01f, RACING_RATE_WIDE = 0.03f;
