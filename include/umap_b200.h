@@ -238,7 +238,7 @@ int umap_knn_last_profile(float* candidate_pass_ms, uint64_t* rows_recomputed, u
  * [offsets[s], offsets[s+1]) of the concatenated arrays (host offsets, u64[n_instances+1],
  * offsets[0] = 0); its kNN ids are local to it (0..n_s-1).  Each instance is validated like
  * learn_manifold (messages prefixed "instance s: ").  Every epoch is one kernel launch over
- * all instances; the SGD task length is autotuned on the first batch of a
+ * all instances; the SGD task length and block shape are autotuned on the first batch of a
  * given size.  The result is an ordinary optimizer handle (step_epochs, embedding,
  * export_edges, schedule_totals, into_fitted work on it; checkpoints do not). */
 int umap_batch_optimizer_new(const umap_config* cfg, uint64_t n_instances, const uint64_t* host_offsets,
